@@ -9,11 +9,20 @@
 // is then re-evaluated once in float-float arithmetic for the reported t
 // and barycentrics.
 //
-// Slab conservativeness: a child plane at p + q*2^e is evaluated as
-// fma(q, 2^e*invd, (p - o)*invd); the rounding error of that expression is
-// below 8u*|invd|*(|p| + 255*2^e + |o|) (u = 2^-24), so the near distance
-// is lowered and the far distance raised by that amount.  Together with
-// outward quantisation this never culls a box the exact ray touches.
+// Slab conservativeness: with s = 2^e, a child plane at p + q*s is evaluated as
+// fma(1 + q/2^15, a, c), a = 2^15*s*invd and c = (p - o)*invd -+ err - a (the
+// byte q becomes the float 1 + q/2^15 by one byte permute, so no conversion or
+// subtraction is needed per child).  With u = 2^-24 and invd within 2u of 1/d (rcp.approx), the
+// rounding errors are below 4u*|invd|*(|p| + |o|) for (p - o)*invd, 3u of its
+// value for the margin, c and the result, 2u*255*s*|invd| for q*s*invd, and
+// 2^15*u*s*|invd| + 2u*255*s*|invd| for c's cancelled term and the last
+// rounding: under |invd|*(7u*(|p| + |o|) + 0.0021*s).  The near distance is
+// lowered and the far distance raised by |invd|*(8u*(|p| + |o|) + 0.00225*s),
+// which widens a box by a quarter of a percent of a grid cell.  Where a
+// overflows (a near-zero direction component in a huge scene) both distances
+// are NaN, which the maxima and minima ignore: that axis does not cull.
+// Together with outward quantisation this never culls a box the exact ray
+// touches.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -59,31 +68,30 @@ __device__ __forceinline__ float min3f(float a, float b, float c) {
 }
 __device__ __forceinline__ float lo32(uint64_t v) { return __uint_as_float((uint32_t)v); }
 __device__ __forceinline__ float hi32(uint64_t v) { return __uint_as_float((uint32_t)(v >> 32)); }
-// (near, far) t of one axis: bytes `sel` of the near / far words as floats (2^23
-// mantissa trick, packed subtraction), then one packed FMA with (adj, adj) and (on, of)
+// (near, far) t of one axis: bytes `sel` of the near / far words become the floats
+// 1 + q / 2^15 (a byte placed in the mantissa), then one packed FMA with (adj, adj) and
+// the offsets
 __device__ __forceinline__ uint64_t slab2(uint32_t nw, uint32_t fw, uint32_t sel, uint64_t adj2, uint64_t off2) {
-  const uint32_t a = __byte_perm(nw, 0x4B000000u, 0x7540u | sel), b = __byte_perm(fw, 0x4B000000u, 0x7540u | sel);
+  const uint32_t a = __byte_perm(nw, 0x3F800000u, 0x7604u | (sel << 4)),
+                 b = __byte_perm(fw, 0x3F800000u, 0x7604u | (sel << 4));
   uint64_t q, t;
-  const uint64_t m = 0x4B0000004B000000ull;  // 2^23, 2^23
   asm("mov.b64 %0, {%1, %2};" : "=l"(q) : "r"(a), "r"(b));
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(q) : "l"(q), "l"(m));
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(t) : "l"(q), "l"(adj2), "l"(off2));
   return t;
 }
 
 struct Slab {
-  float adj, on, of;  // q scale, near offset, far offset
+  float adj, on, of;  // scale, near and far offset for the factor 1 + q / 2^15
 };
 
 __device__ __forceinline__ Slab make_slab(float p, float e_bits, float inv, float o) {
-  float s = e_bits;                 // 2^e
-  float adj = s * inv;
-  float org = (p - o) * inv;
-  float err = 4.76837158203125e-7f * fabsf(inv) * (fabsf(p) + 255.0f * s + fabsf(o));  // 8u
+  const float s = e_bits;                 // 2^e
+  const float org = (p - o) * inv;
+  const float err = fabsf(inv) * fmaf(2.25e-3f, s, 4.76837158203125e-7f * (fabsf(p) + fabsf(o)));
   Slab r;
-  r.adj = adj;
-  r.on = org - err;
-  r.of = org + err;
+  r.adj = s * (32768.0f * inv);
+  r.on = (org - err) - r.adj;
+  r.of = (org + err) - r.adj;
   return r;
 }
 
@@ -98,12 +106,19 @@ struct LaneRay {
 // Per-ray traversal constants for origin o and direction d (world ray, or an
 // instance's local ray: d is not renormalised, so t is the same in both).  The
 // origin and direction are kept once, in the watertight test's state.
-__device__ __forceinline__ void set_ray(LaneRay& R, WtRay& wr, float ox, float oy, float oz, float dx, float dy,
+__device__ __forceinline__ void set_ray(LaneRay& R, TravRay& wr, float ox, float oy, float oz, float dx, float dy,
                                         float dz) {
-  auto safe = [](float d) { return fabsf(d) > 1e-30f ? d : copysignf(1e-30f, d); };
-  R.ix = __frcp_rn(safe(dx)); R.iy = __frcp_rn(safe(dy)); R.iz = __frcp_rn(safe(dz));
+  // a component below 1e-30 of the largest is taken as that (a drift far inside
+  // the slab margins); never a subnormal, whose reciprocal overflows
+  const float least = fmaxf(1e-30f * max3f(fabsf(dx), fabsf(dy), fabsf(dz)), 1.17549435e-38f);
+  auto inverse = [least](float d) {
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(fabsf(d) > least ? d : copysignf(least, d)));
+    return r;
+  };
+  R.ix = inverse(dx); R.iy = inverse(dy); R.iz = inverse(dz);
   R.oct = (R.ix < 0.0f ? 4u : 0u) | (R.iy < 0.0f ? 2u : 0u) | (R.iz < 0.0f ? 1u : 0u);
-  wr = wt_setup(ox, oy, oz, dx, dy, dz);
+  wr = trav_setup(ox, oy, oz, dx, dy, dz);
 }
 
 // Reorders an 8-bit slot mask into key order: bit s moves to bit s ^ oct.
@@ -122,23 +137,23 @@ __device__ __forceinline__ uint32_t nibble_spread8(uint32_t m) {
   return m * 15u;
 }
 
-// Resident CTAs per SM the register budget is cut for: 8 (64 registers, some
-// L1-cached spills) for single-level trees, 6 (80 registers) for two-level
-// scenes, whose instance state spills several times more at 64 -- measured:
-// box room 4 % faster at 8, instanced cloud 7 % slower at 8.
-template <bool TWO>
-constexpr int trace_min_blocks() { return TWO ? 6 : 8; }
+// Resident CTAs per SM the register budget is cut for (80 registers, spills
+// only around the out-of-line exact test).  Measured (B200) at 5 / 6 / 7 / 8 /
+// 9: the 1,048,576-ray query 1.01 / 0.98 / 1.01 / 1.14 / 1.42 ms, the box-room
+// frame 25.9 / 24.8 / 25.1 / 25.9 / 28.4 ms; the instanced frame 24.7 / 24.7 /
+// 25.5 ms at 5 / 6 / 7.
+constexpr int kTraceBlocks = 6;
 
-// Watertight tests per loop iteration, at most.  Measured (B200, CUDA events):
-// single-level trees one (box room 512^2 x 64 spp frame 30.7 -> 28.5 ms, its
-// closest-hit traces 18.5 -> 16.4 ms; the 1,048,576-ray query 1.25 -> 1.19 ms;
-// three: 31.1 ms and 1.41 ms), two-level scenes two (the instanced cloud's
-// frame 30.6 ms against 30.7 with one and 32.0 with three).
-template <bool TWO>
-__host__ __device__ constexpr int tri_per_step() { return TWO ? 2 : 1; }
+// Idle lanes a warp gathers before it refills them.  Setting a ray up costs
+// about as much as expanding a node and a warp of the box-room frame finishes
+// 4.4 rays per iteration: refilling every idle lane at once ran the set-up in
+// 94 % of the iterations for those few lanes.  Measured at 1 / 4 / 6 / 8 / 12:
+// box-room frame 27.2 / 26.3 / 26.0 / 25.9 / 26.1 ms, query 1.18 / 1.13 / 1.13 /
+// 1.14 / 1.16 ms (at 64 registers).
+constexpr int kRefillLanes = 8;
 
 template <bool ANY, bool TWO, bool HOT>
-__global__ void __launch_bounds__(kBlock, trace_min_blocks<TWO>())
+__global__ void __launch_bounds__(kBlock, kTraceBlocks)
     k_trace(const uint4* __restrict__ nodes, const float4* __restrict__ tris,
                                                   const float4* __restrict__ rays, size_t n,
                                                   int4* __restrict__ hits, uint8_t* __restrict__ occluded,
@@ -151,12 +166,12 @@ __global__ void __launch_bounds__(kBlock, trace_min_blocks<TWO>())
                                                   const uint32_t* __restrict__ order,
                                                   const float4* __restrict__ inst_table) {
   // Persistent warps, one ray per lane.  Every iteration each live lane
-  // (1) expands at most one wide node, (2) runs at most tri_per_step()
-  // watertight triangle tests from a two-entry queue of triangle groups, and (3) picks
+  // (1) expands at most one wide node, (2) runs at most one watertight
+  // triangle test from a two-entry queue of triangle groups, and (3) picks
   // its next node without waiting for its queued triangles.  Node work and
   // triangle work therefore proceed in lock-step phases with most lanes
   // busy in each, and a lane whose ray finished takes the next unclaimed
-  // ray from its warp's pool (one atomicAdd per 16 rays).
+  // ray from its warp's pool (one atomicAdd per kChunk rays).
   // The group stack is a per-thread local array: the hardware interleaves it
   // across the warp, it is cached in L1 only where it is touched (rays rarely
   // go deep), and no shared memory is reserved for it, so the SM keeps its
@@ -198,14 +213,15 @@ __global__ void __launch_bounds__(kBlock, trace_min_blocks<TWO>())
   constexpr uint32_t kInstGroup = 0x40000000u;
   constexpr uint32_t kTagMask = 0xC0000000u;
   // rays per pool refill: small enough to spread short launches over all warps
-  // (two-level: 16), 32 for single-level trees (box room 0.8 % faster than 16)
-  constexpr uint32_t kChunk = TWO ? 16 : 32;
+  // (16 / 32 / 64: instanced frame 25.1 / 24.7 / 25.7 ms, box room 26.7 / 25.9 /
+  // 25.5 ms, a 1,000-ray query 55 / 54 / 98 us)
+    constexpr uint32_t kChunk = 32;
 
   bool live = false, exhausted = false;
   uint32_t ray = 0, pool_next = 0, pool_end = 0;
   const uint32_t n32 = n_dev ? *n_dev : (uint32_t)n;
   LaneRay R;
-  WtRay wr;
+  TravRay wr;
   float wox = 0.f, woy = 0.f, woz = 0.f, wdx = 0.f, wdy = 0.f, wdz = 0.f;  // world ray (two-level)
   int cur_inst = -1, best_inst = -1;
   uint32_t cur_flags = 0;  // material flags of the instance being traversed (two-level)
@@ -217,7 +233,8 @@ __global__ void __launch_bounds__(kBlock, trace_min_blocks<TWO>())
   while (true) {
     // ---- refill idle lanes from the warp's ray pool
     const uint32_t idle = __ballot_sync(kFull, !live);
-    if (idle) {
+    // (a warp whose pool is spent only counts them; the last lane to finish ends it)
+    if (idle == kFull || (__popc(idle) >= kRefillLanes && !(exhausted && pool_next >= pool_end))) {
       if (pool_next >= pool_end && !exhausted) {
         unsigned long long base = 0;
         if (lane == 0) base = atomicAdd(ray_counter, (unsigned long long)kChunk);
@@ -327,23 +344,26 @@ __global__ void __launch_bounds__(kBlock, trace_min_blocks<TWO>())
             const uint32_t tri = w1.y + (uint32_t)(__ffs(th) - 1);
             th &= th - 1;
             const float4* rec = tris + 4 * (size_t)tri;
-            const float4 a = __ldg(rec), b = __ldg(rec + 1), c = __ldg(rec + 2);
-            const uint32_t fl = __float_as_uint(c.w) | cur_flags;
+            const uint32_t fl = __float_as_uint(__ldg(rec + 2).w) | cur_flags;
             if (ANY && (fl & VT_MATERIAL_NO_SHADOW)) continue;
-            const float t = wt_candidate(wr, make_float3(a.x, a.y, a.z), make_float3(b.x, b.y, b.z),
-                                         make_float3(c.x, c.y, c.z), R.tmin, R.closest,
-                                         [rec] { return __ldg(rec + 3); }, (fl & VT_MATERIAL_SINGLE_SIDED) != 0);
+            const float t = trav_exact(wr.o[0], wr.o[1], wr.o[2], wr.d[0], wr.d[1], wr.d[2], rec, fmaxf(R.tmin, 0.0f),
+                                       R.closest, (fl & VT_MATERIAL_SINGLE_SIDED) != 0);
             if (t >= 0.0f) { R.closest = t; R.best = (int)tri; best_inst = cur_inst; }
           }
         }
       }
     }
 
-    // ---- (2) triangle tests from the queue head: one per iteration for
-    // single-level trees, two for two-level scenes (see kTriPerStep)
+    // ---- (2) one triangle test from the queue head.  Measured: two a step made
+    // the query 4 % faster and the box-room frame 4 % slower; running the phase
+    // only once 8 lanes want it or 4 wait for it, two tests at a time, made the
+    // box room 3 % faster and the query and the instanced frame 4-6 % slower.
+    // (A loop, so that the compiler brings the lanes together again behind it:
+    // with a plain branch the lanes went on apart, 25 % slower; __syncwarp
+    // between the phases, 20 %.)
     bool done = false;
 #pragma unroll 1
-    for (int rep = 0; rep < tri_per_step<TWO>(); ++rep) {
+    for (int rep = 0; rep < 1; ++rep) {
       if (q0m == 0) break;
       const uint32_t tri = q0b + (uint32_t)(__ffs(q0m) - 1);
       q0m &= q0m - 1;
@@ -351,15 +371,14 @@ __global__ void __launch_bounds__(kBlock, trace_min_blocks<TWO>())
       const float4* rec = tris + 4 * (size_t)tri;
       const float4 a = __ldg(rec), b = __ldg(rec + 1), c = __ldg(rec + 2);
       const uint32_t fl = __float_as_uint(c.w) | cur_flags;
-      if (ANY && (fl & VT_MATERIAL_NO_SHADOW)) continue;
-      const float t = wt_candidate(wr, make_float3(a.x, a.y, a.z), make_float3(b.x, b.y, b.z),
-                                   make_float3(c.x, c.y, c.z), R.tmin, R.closest, [rec] { return __ldg(rec + 3); },
-                                   (fl & VT_MATERIAL_SINGLE_SIDED) != 0);
-      if (t >= 0.0f) {
-        R.closest = t;
-        R.best = (int)tri;
-        best_inst = cur_inst;
-        if (ANY) { done = true; break; }
+      if (!(ANY && (fl & VT_MATERIAL_NO_SHADOW))) {
+        const float t = wt_candidate(wr, rec, a, b, c, R.tmin, R.closest, (fl & VT_MATERIAL_SINGLE_SIDED) != 0);
+        if (t >= 0.0f) {
+          R.closest = t;
+          R.best = (int)tri;
+          best_inst = cur_inst;
+          if (ANY) done = true;
+        }
       }
     }
 
