@@ -231,7 +231,8 @@ vt_status vt_bvh_build_device(int32_t device, const float* d_positions, size_t p
     b->ntri = (int64_t)(index_words / b->opts.index_stride);
     BinaryBvhDevice td;
     if (separate_tree(b->opts))
-      build_binary_gpu(d_positions, position_words, d_indices, index_words, traversal_options(b->opts), s, &td);
+      build_binary_gpu(d_positions, position_words, d_indices, index_words, traversal_options(b->opts), s, &td,
+                       false);
     WideBvhDevice wd;
     const WideBvhHost w = encode_wide_gpu(separate_tree(b->opts) ? td : bd, d_positions, b->opts.position_stride,
                                           d_indices, b->opts.index_stride, nullptr, 0, 0, query_collapse(b->opts),

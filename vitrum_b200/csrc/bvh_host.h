@@ -68,9 +68,12 @@ struct BinaryBvhDevice {
   size_t n_nodes = 0, ntri = 0;
 };
 // The same tree built on the GPU from device positions / indices; with keep,
-// its device arrays are handed over for a device encoding.
+// its device arrays are handed over for a device encoding (nodes: capacity for
+// 2 per triangle, n_nodes in use); without host_copy the returned nodes and
+// order stay empty.
 BinaryBvhHost build_binary_gpu(const float* d_pos, size_t position_words, const uint32_t* d_idx, size_t index_words,
-                               const BuildOptions& o, cudaStream_t s, BinaryBvhDevice* keep = nullptr);
+                               const BuildOptions& o, cudaStream_t s, BinaryBvhDevice* keep = nullptr,
+                               bool host_copy = true);
 
 // Binned-SAH binary build on host arrays (throws vt::Error).
 BinaryBvhHost build_binary_host(const float* positions, size_t position_words, const uint32_t* indices,
