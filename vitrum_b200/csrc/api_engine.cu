@@ -62,8 +62,8 @@ struct vt_engine {
   // scene
   bool has_scene = false;
   vt::BinaryBvhHost binary;
-  DeviceBuffer<uint4> nodes;
-  DeviceBuffer<float4> tris;
+  vt::PoolBuffer<uint4> nodes;
+  vt::PoolBuffer<float4> tris;
   int wide_depth = 1;
   int stack_depth = 16;            // traversal stack entries the scene needs
   DeviceBuffer<float4> insts;      // instance records in top-level leaf order
@@ -186,6 +186,7 @@ static vt::SceneBuild scene_build_of(const vt_engine* e) {
   sb.device = e->device;
   sb.stream = e->stream;
   sb.validate = e->opts.debug != 0;
+  sb.keep = true;
   sb.bvh_width = e->opts.bvh_width;
   return sb;
 }
@@ -199,17 +200,22 @@ void set_scene(vt_engine* e, const vt_scene_desc* sc) {
   vt::PackedScene p = vt::pack_scene(sc, 0, 0, e->opts.bvh_max_leaf, scene_build_of(e));
   cudaStream_t s = e->stream;
   struct Staged {
-    DeviceBuffer<uint4> nodes;
-    DeviceBuffer<float4> tris, insts, inst_table, inst_l2w;
+    vt::PoolBuffer<uint4> nodes;
+    vt::PoolBuffer<float4> tris;
+    DeviceBuffer<float4> insts, inst_table, inst_l2w;
     DeviceBuffer<vt::pt::Material> materials;
     DeviceBuffer<float4> emitters, points, area_lights, dirs, env;
     DeviceBuffer<float> emitter_cdf, env_marginal, env_conditional, light_tree;
   } n;
-  n.nodes.resize(p.node_words.size() / 4);
-  VT_CUDA(cudaMemcpyAsync(n.nodes.ptr, p.node_words.data(), p.node_words.size() * 4, cudaMemcpyHostToDevice, s));
-  n.tris.resize(std::max<size_t>(p.rec_floats.size() / 4, 1));
-  if (!p.rec_floats.empty())
-    VT_CUDA(cudaMemcpyAsync(n.tris.ptr, p.rec_floats.data(), p.rec_floats.size() * 4, cudaMemcpyHostToDevice, s));
+  // a single-level tree built on the GPU stays there (of the box room's 262,146
+  // triangles the way over the host took 27 of set_scene's 40 ms)
+  const size_t n_u4 = p.on_device ? 5 * p.dev.n_nodes : p.node_words.size() / 4;
+  const size_t r_f4 = p.on_device ? 4 * p.dev.n_recs : p.rec_floats.size() / 4;
+  const cudaMemcpyKind kind = p.on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+  n.nodes.resize(n_u4, s);
+  VT_CUDA(cudaMemcpyAsync(n.nodes.ptr, p.on_device ? p.dev.nodes.ptr : p.node_words.data(), n_u4 * 16, kind, s));
+  n.tris.resize(std::max<size_t>(r_f4, 1), s);
+  if (r_f4) VT_CUDA(cudaMemcpyAsync(n.tris.ptr, p.on_device ? p.dev.recs.ptr : p.rec_floats.data(), r_f4 * 16, kind, s));
   const bool two_level = p.two_level;
   std::vector<float4> il(p.inst_lanes.size() / 4), it(p.inst_tab.size() / 4), ir(p.inst_rows.size() / 4);
   if (!il.empty()) std::memcpy(il.data(), p.inst_lanes.data(), p.inst_lanes.size() * 4);
@@ -334,7 +340,8 @@ void update_instances(vt_engine* e, const vt_instance_desc* insts, size_t n, boo
   e->drop_graphs();
   const size_t blas_u4 = (size_t)e->tlas_root * 5, tlas_u4 = tw.nodes.size() / 4;
   if (blas_u4 + tlas_u4 != e->nodes.count) {
-    DeviceBuffer<uint4> grown(blas_u4 + tlas_u4);
+    vt::PoolBuffer<uint4> grown;
+    grown.resize(blas_u4 + tlas_u4, s);
     if (blas_u4)
       VT_CUDA(cudaMemcpyAsync(grown.ptr, e->nodes.ptr, blas_u4 * sizeof(uint4), cudaMemcpyDeviceToDevice, s));
     VT_CUDA(cudaStreamSynchronize(s));
@@ -412,9 +419,9 @@ void update_mesh(vt_engine* e, size_t m, const vt_mesh_desc* md, bool rebuild) {
   VT_CUDA(cudaStreamSynchronize(s));
   e->drop_graphs();
   const size_t blas_u4 = e->blas_words.size() / 4;
-  e->nodes.resize(blas_u4 + tlas_u4);  // the top level's part is written by update_instances
+  e->nodes.resize(blas_u4 + tlas_u4, s);  // the top level's part is written by update_instances
   VT_CUDA(cudaMemcpyAsync(e->nodes.ptr, e->blas_words.data(), e->blas_words.size() * 4, cudaMemcpyHostToDevice, s));
-  e->tris.resize(std::max<size_t>(e->rec_host.size() / 4, 1));
+  e->tris.resize(std::max<size_t>(e->rec_host.size() / 4, 1), s);
   VT_CUDA(cudaMemcpyAsync(e->tris.ptr, e->rec_host.data(), e->rec_host.size() * 4, cudaMemcpyHostToDevice, s));
   VT_CUDA(cudaStreamSynchronize(s));
   e->view.tris = e->tris.ptr;

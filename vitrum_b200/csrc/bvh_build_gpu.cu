@@ -1089,8 +1089,8 @@ BinaryBvhHost build_binary_gpu(const float* d_pos, size_t position_words, const 
   w.bins[1] = reinterpret_cast<uint32_t*>(mem.ptr + at_b1);
   w.small = reinterpret_cast<uint32_t*>(mem.ptr + at_small);
   w.temp = reinterpret_cast<BinaryNode*>(mem.ptr + at_temp);
-  DeviceBuffer<uint32_t> order(ntri);
-  DeviceBuffer<BinaryNode> dout(2 * ntri);
+  ScratchBuffer<uint32_t> order(ntri, s);
+  ScratchBuffer<BinaryNode> dout(2 * ntri, s);
   const size_t small_smem = sizeof(Small) + (size_t)(kSmallThreads / 32) * 14 * o.bins * 4;
   static bool attr = false;
   if (!attr) {

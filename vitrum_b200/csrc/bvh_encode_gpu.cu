@@ -365,6 +365,7 @@ struct EmitArgs {
   const uint32_t* idx;       // triangles: indices (stride is)
   int is;
   const uint32_t* tri_mat;   // optional, one per source triangle
+  const uint32_t* mat_flags; // optional, one per material: flags word of its records
   const float* inst_recs;    // top level: 16 floats per instance (else null)
   uint32_t node_base, rec_base;
 };
@@ -458,6 +459,7 @@ __global__ void k_level_emit(EmitArgs A, const uint32_t* __restrict__ level, uin
         rec[13] = nn[1];
         rec[14] = nn[2];
         rec[15] = valid ? 1.0f : 0.0f;
+        if (valid && A.mat_flags && A.tri_mat) rec[11] = __uint_as_float(A.mat_flags[A.tri_mat[src]]);
       }
     } else {
       imask |= (uint8_t)(1u << s);
@@ -476,7 +478,8 @@ __global__ void k_level_emit(EmitArgs A, const uint32_t* __restrict__ level, uin
 
 WideBvhHost encode_wide_gpu(const BinaryBvhDevice& bin, const float* d_pos, int pos_stride, const uint32_t* d_idx,
                             int idx_stride, const uint32_t* d_tri_mat, uint32_t node_base, uint32_t rec_base,
-                            const WideCollapse* sah, const float* d_inst_recs, cudaStream_t s, WideBvhDevice* keep) {
+                            const WideCollapse* sah, const float* d_inst_recs, cudaStream_t s, WideBvhDevice* keep,
+                            bool host_copy, const uint32_t* d_mat_flags) {
   WideBvhHost out;
   const uint32_t n = (uint32_t)bin.n_nodes;
   if (bin.ntri == 0 || n == 0) {
@@ -486,11 +489,12 @@ WideBvhHost encode_wide_gpu(const BinaryBvhDevice& bin, const float* d_pos, int 
     out.nodes.assign(w, w + 20);
     out.depth = 1;
     if (keep) {
-      keep->nodes.resize(20);
+      keep->nodes.resize(20, s);
       VT_CUDA(cudaMemcpyAsync(keep->nodes.ptr, w, sizeof w, cudaMemcpyHostToDevice, s));
-      keep->recs.resize(0);
+      keep->recs.resize(0, s);
       keep->n_nodes = 1;
       keep->n_recs = 0;
+      keep->depth = 1;
       VT_CUDA(cudaStreamSynchronize(s));
     }
     return out;
@@ -512,9 +516,9 @@ WideBvhHost encode_wide_gpu(const BinaryBvhDevice& bin, const float* d_pos, int 
   }
   // wide nodes: at most one per binary interior node (a lone leaf root: one)
   const uint32_t max_wide = n / 2 + 1;
-  DeviceBuffer<uint32_t> words((size_t)20 * max_wide);
+  ScratchBuffer<uint32_t> words((size_t)20 * max_wide, s);
   size_t rec_cap = 28 + 4 * (size_t)bin.ntri + 64;
-  DeviceBuffer<float> recs(16 * rec_cap);
+  ScratchBuffer<float> recs(16 * rec_cap, s);
   VT_CUDA(cudaMemsetAsync(recs.ptr, 0, recs.bytes(), s));
   ScratchBuffer<uint32_t> lvl_a(max_wide, s), lvl_b(max_wide, s), n_int(max_wide, s), span(max_wide, s);
   ScratchBuffer<LevelPlan> plan(max_wide, s);
@@ -524,7 +528,7 @@ WideBvhHost encode_wide_gpu(const BinaryBvhDevice& bin, const float* d_pos, int 
   const uint32_t root = 0;
   VT_CUDA(cudaMemcpyAsync(lvl_a.ptr, &root, sizeof root, cudaMemcpyHostToDevice, s));
   EmitArgs A{bin.nodes.ptr, sah ? dp.ptr : nullptr, bin.order.ptr, d_pos, pos_stride, d_idx, idx_stride, d_tri_mat,
-             d_inst_recs, node_base, rec_base};
+             d_mat_flags, d_inst_recs, node_base, rec_base};
   uint32_t level_n = 1, level_start = 0, rec_used = 28;
   int depth = 0;
   ScratchBuffer<uint32_t>* cur = &lvl_a;
@@ -544,7 +548,7 @@ WideBvhHost encode_wide_gpu(const BinaryBvhDevice& bin, const float* d_pos, int 
     if (rec_used + tot[1] > rec_cap) {
       // grow the record array (more leaf slots than the first estimate)
       const size_t cap = std::max<size_t>(rec_used + tot[1] + 64, rec_cap * 3 / 2);
-      DeviceBuffer<float> bigger(16 * cap);
+      ScratchBuffer<float> bigger(16 * cap, s);
       VT_CUDA(cudaMemsetAsync(bigger.ptr, 0, bigger.bytes(), s));
       VT_CUDA(cudaMemcpyAsync(bigger.ptr, recs.ptr, 16 * sizeof(float) * rec_used, cudaMemcpyDeviceToDevice, s));
       recs = std::move(bigger);
@@ -563,16 +567,19 @@ WideBvhHost encode_wide_gpu(const BinaryBvhDevice& bin, const float* d_pos, int 
   VT_CUDA(cudaStreamSynchronize(s));
   if (bad) fail(VT_ERR_BUILD, "leaf records exceed 2^30");
   out.depth = depth;
-  out.nodes.resize((size_t)20 * level_start);
-  out.tris.resize((size_t)16 * rec_used);
-  VT_CUDA(cudaMemcpyAsync(out.nodes.data(), words.ptr, out.nodes.size() * 4, cudaMemcpyDeviceToHost, s));
-  VT_CUDA(cudaMemcpyAsync(out.tris.data(), recs.ptr, out.tris.size() * 4, cudaMemcpyDeviceToHost, s));
-  VT_CUDA(cudaStreamSynchronize(s));
+  if (host_copy) {
+    out.nodes.resize((size_t)20 * level_start);
+    out.tris.resize((size_t)16 * rec_used);
+    VT_CUDA(cudaMemcpyAsync(out.nodes.data(), words.ptr, out.nodes.size() * 4, cudaMemcpyDeviceToHost, s));
+    VT_CUDA(cudaMemcpyAsync(out.tris.data(), recs.ptr, out.tris.size() * 4, cudaMemcpyDeviceToHost, s));
+    VT_CUDA(cudaStreamSynchronize(s));
+  }
   if (keep) {
     keep->nodes = std::move(words);
     keep->recs = std::move(recs);
     keep->n_nodes = level_start;
     keep->n_recs = rec_used;
+    keep->depth = depth;
   }
   return out;
 }

@@ -63,8 +63,8 @@ WideProof validate_wide(const uint32_t* nodes, size_t n_nodes, const float* recs
 // Device copies of a binary tree: nodes in preorder and the BVH-order
 // triangle permutation (reordered_to_source).
 struct BinaryBvhDevice {
-  DeviceBuffer<BinaryNode> nodes;
-  DeviceBuffer<uint32_t> order;
+  ScratchBuffer<BinaryNode> nodes;
+  ScratchBuffer<uint32_t> order;
   size_t n_nodes = 0, ntri = 0;
 };
 // The same tree built on the GPU from device positions / indices; with keep,
@@ -92,20 +92,32 @@ struct WideCollapse {
 };
 
 // Device copies of an encoded tree: 20 words per wide node, 16 floats per record.
+// (the arrays hold at least n_nodes and n_recs of them).
 struct WideBvhDevice {
-  DeviceBuffer<uint32_t> nodes;
-  DeviceBuffer<float> recs;
+  ScratchBuffer<uint32_t> nodes;
+  ScratchBuffer<float> recs;
   size_t n_nodes = 0, n_recs = 0;
+  int depth = 0;
 };
 // encode_wide on the GPU from a device binary tree (bvh_encode_gpu.cu): the
 // same node words and records.  Triangle records from d_pos / d_idx (and
 // d_tri_mat), or, with d_inst_recs (16 floats per instance), a top level's
-// instance records; sah == nullptr: the reference's greedy collapse.  The
-// result is returned on the host; with keep also kept on the device.
+// instance records; sah == nullptr: the reference's greedy collapse.  With
+// d_mat_flags (one word per material) each valid triangle record carries its
+// material's flags.  The result is returned on the host (host_copy; else only
+// its depth) and, with keep, kept on the device.
 WideBvhHost encode_wide_gpu(const BinaryBvhDevice& bin, const float* d_pos, int pos_stride, const uint32_t* d_idx,
                             int idx_stride, const uint32_t* d_tri_mat, uint32_t node_base, uint32_t rec_base,
                             const WideCollapse* sah, const float* d_inst_recs, cudaStream_t s,
-                            WideBvhDevice* keep = nullptr);
+                            WideBvhDevice* keep = nullptr, bool host_copy = true,
+                            const uint32_t* d_mat_flags = nullptr);
+
+// The structural proofs of validate_binary and validate_wide (triangle trees,
+// bases 0) on device arrays (bvh_prove_gpu.cu); a tree that fails is copied to
+// the host, whose proof names the violation.  Throws vt::Error(VT_ERR_BUILD).
+void prove_binary_gpu(const BinaryNode* d_nodes, size_t n_nodes, size_t ntri, int stack_cap, cudaStream_t s);
+void prove_wide_gpu(const uint32_t* d_words, size_t n_nodes, const float* d_recs, size_t n_recs, size_t n_items,
+                    int stack_cap, cudaStream_t s);
 
 // tri_materials (optional, one per source triangle) is stored in each record's v1.w.
 // node_base / rec_base offset the encoded indices for trees concatenated into shared arrays.

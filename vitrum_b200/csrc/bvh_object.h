@@ -14,14 +14,13 @@ struct vt_bvh {
   int device = 0;
   vt::BuildOptions opts;
   vt::BinaryBvhHost binary;              // binary tree in the reference layout (for export)
-  vt::DeviceBuffer<uint4> nodes;         // 8-wide nodes
-  vt::DeviceBuffer<float4> tris;         // triangle records
-  vt::DeviceBuffer<int> status;          // traversal status word
-  vt::DeviceBuffer<unsigned long long> counter;  // persistent-kernel ray counter (calls on one bvh are serialised)
-  std::vector<uint32_t> wide_host_nodes;  // the published 8-wide nodes and records (host copies, for export)
-  std::vector<float> wide_host_recs;
+  vt::PoolBuffer<uint4> nodes;           // 8-wide nodes
+  vt::PoolBuffer<float4> tris;           // triangle records (at least one allocated)
+  vt::PoolBuffer<int> status;            // traversal status word
+  vt::PoolBuffer<unsigned long long> counter;  // persistent-kernel ray counter (calls on one bvh are serialised)
   int64_t ntri = 0;
-  int64_t wide_count = 0;
+  int64_t wide_count = 0;                // 8-wide nodes
+  int64_t rec_count = 0;                 // triangle records
   int wide_depth = 0;
   double build_ms = 0.0;
   // staging for the host-buffer entry points

@@ -167,31 +167,39 @@ void append_mesh(const vt_mesh_desc& md, size_t m, size_t material_count, std::v
   if ((md.vertex_count && !md.positions) || (md.triangle_count && !md.indices))
     fail(VT_ERR_INVALID_ARGUMENT, "mesh " + std::to_string(m) + " has null arrays");
   const uint32_t base = (uint32_t)(pos.size() / 4);
-  for (size_t v = 0; v < md.vertex_count; ++v) {
+  const size_t tri0 = idx.size() / 4;
+  pos.resize(4 * ((size_t)base + md.vertex_count));
+  idx.resize(4 * (tri0 + md.triangle_count));
+  tri_mat.resize(tri_mat.size() + md.triangle_count, md.material);
+  float* p = pos.data() + 4 * (size_t)base;
+  for (size_t v = 0; v < md.vertex_count; ++v, p += 4) {
     for (int k = 0; k < 3; ++k) {
       const float x = md.positions[3 * v + k];
       if (!std::isfinite(x)) fail(VT_ERR_RANGE, "mesh " + std::to_string(m) + " has a non-finite position");
-      pos.push_back(x);
+      p[k] = x;
     }
-    pos.push_back(0.0f);
+    p[3] = 0.0f;
   }
-  for (size_t t = 0; t < md.triangle_count; ++t) {
+  uint32_t* q = idx.data() + 4 * tri0;
+  for (size_t t = 0; t < md.triangle_count; ++t, q += 4) {
     for (int k = 0; k < 3; ++k) {
       const uint32_t i = md.indices[3 * t + k];
       if (i >= md.vertex_count) fail(VT_ERR_RANGE, "mesh " + std::to_string(m) + " index out of range");
-      idx.push_back(base + i);
+      q[k] = base + i;
     }
-    idx.push_back(0u);
-    tri_mat.push_back(md.material);
+    q[3] = 0u;
   }
 }
 
 // The engine's tree over vertices pos (4 floats each) and triangles idx (4
 // u32 each): the binned-SAH build and the SAH-optimal 8-wide encoding, on the
-// GPU or on the host (the same words either way).
+// GPU or on the host (the same words either way).  With dev (GPU builds), the
+// tree stays there, its records carrying their materials' flags, and bin holds
+// the root alone.
 static void build_tree(const SceneBuild& sb, const std::vector<float>& pos, const std::vector<uint32_t>& idx,
                        const uint32_t* tri_mat, uint32_t node_base, uint32_t rec_base, int max_leaf,
-                       BinaryBvhHost& bin, WideBvhHost& wide) {
+                       BinaryBvhHost& bin, WideBvhHost& wide, WideBvhDevice* dev = nullptr,
+                       const std::vector<uint32_t>* mat_flags = nullptr) {
   BuildOptions bo;
   bo.max_leaf = max_leaf;
   bo.bins = kEngineBins;
@@ -206,9 +214,19 @@ static void build_tree(const SceneBuild& sb, const std::vector<float>& pos, cons
     if (!idx.empty()) VT_CUDA(cudaMemcpyAsync(didx.ptr, idx.data(), idx.size() * 4, cudaMemcpyHostToDevice, sb.stream));
     if (ntri && tri_mat) VT_CUDA(cudaMemcpyAsync(dmat.ptr, tri_mat, ntri * 4, cudaMemcpyHostToDevice, sb.stream));
     BinaryBvhDevice bd;
-    bin = build_binary_gpu(dpos.ptr, pos.size(), didx.ptr, idx.size(), bo, sb.stream, &bd);
+    bin = build_binary_gpu(dpos.ptr, pos.size(), didx.ptr, idx.size(), bo, sb.stream, &bd, dev == nullptr);
+    ScratchBuffer<uint32_t> dflags;
+    if (dev && mat_flags && !mat_flags->empty()) {
+      dflags.resize(mat_flags->size(), sb.stream);
+      VT_CUDA(cudaMemcpyAsync(dflags.ptr, mat_flags->data(), dflags.bytes(), cudaMemcpyHostToDevice, sb.stream));
+    }
     wide = encode_wide_gpu(bd, dpos.ptr, 4, didx.ptr, 4, tri_mat ? dmat.ptr : nullptr, node_base, rec_base,
-                           &collapse, nullptr, sb.stream);
+                           &collapse, nullptr, sb.stream, dev, dev == nullptr, dflags.ptr);
+    if (dev && bd.n_nodes) {
+      bin.nodes.resize(1);
+      VT_CUDA(cudaMemcpyAsync(bin.nodes.data(), bd.nodes.ptr, sizeof(BinaryNode), cudaMemcpyDeviceToHost, sb.stream));
+      VT_CUDA(cudaStreamSynchronize(sb.stream));
+    }
   } else {
     bin = build_binary_host(pos.data(), pos.size(), idx.data(), idx.size(), bo);
     wide = encode_wide(bin, pos.data(), 4, idx.data(), 4, tri_mat, node_base, rec_base, &collapse);
@@ -233,8 +251,8 @@ WideBvhHost encode_top_level(const SceneBuild& sb, const BinaryBvhHost& tl, cons
   BinaryBvhDevice bd;
   bd.n_nodes = tl.nodes.size();
   bd.ntri = tl.reordered_to_source.size();
-  bd.nodes.resize(std::max<size_t>(bd.n_nodes, 1));
-  bd.order.resize(std::max<size_t>(bd.ntri, 1));
+  bd.nodes.resize(std::max<size_t>(bd.n_nodes, 1), sb.stream);
+  bd.order.resize(std::max<size_t>(bd.ntri, 1), sb.stream);
   ScratchBuffer<float> drecs(std::max<size_t>(16 * recs.size(), 1), sb.stream);
   if (bd.n_nodes)
     VT_CUDA(cudaMemcpyAsync(bd.nodes.ptr, tl.nodes.data(), bd.n_nodes * sizeof(BinaryNode), cudaMemcpyHostToDevice,
@@ -309,7 +327,11 @@ PackedScene pack_scene(const vt_scene_desc* sc, uint32_t node_base, uint32_t rec
   uint32_t root = 0;
   if (!two_level) {
     WideBvhHost w;
-    build_tree(sb, pos, idx, tri_mat.data(), node_base, rec_base, max_leaf, p.binary, w);
+    p.on_device = sb.gpu && sb.keep && !sb.validate;
+    std::vector<uint32_t> flags(mats.size());
+    for (size_t i = 0; i < mats.size(); ++i) flags[i] = mats[i].flags;
+    build_tree(sb, pos, idx, tri_mat.data(), node_base, rec_base, max_leaf, p.binary, w, p.on_device ? &p.dev : nullptr,
+               &flags);
     node_words = std::move(w.nodes);
     rec_floats = std::move(w.tris);
     depth = w.depth;

@@ -38,6 +38,10 @@ struct PackedScene {
   float env_rotation = 0.0f;
   std::vector<float> light_tree;     // packed light tree over the light entries (two or more entries)
   size_t ntri = 0;
+  // SceneBuild::keep: the single-level tree on the device; node_words and
+  // rec_floats are empty then, and of the binary tree only the root is here
+  bool on_device = false;
+  WideBvhDevice dev;
   // two-level: per mesh its bottom-level root node and local bounds; the deepest bottom level
   std::vector<uint32_t> blas_root;
   std::vector<std::array<double, 6>> local_box;
@@ -63,6 +67,7 @@ struct SceneBuild {
   int device = 0;
   cudaStream_t stream = nullptr;
   bool validate = true;
+  bool keep = false;  // GPU builds of single-level scenes leave the tree on the device (PackedScene::dev)
   int bvh_width = 8;  // children per wide node at most of the triangle trees (2..8)
 };
 BlasPack pack_blas(const std::vector<float>& pos, const std::vector<uint32_t>& idx, uint32_t material,

@@ -466,7 +466,7 @@ BinaryBvhHost build_tlas_gpu(const double* aabbs, size_t n, int max_leaf, int bi
   }
   ScratchBuffer<double> d_aabbs(6 * n, s), mn(3 * n, s), mx(3 * n, s), cen(3 * n, s), skey(2 * n, s),
       nmn(3 * 2 * n, s), nmx(3 * 2 * n, s);
-  DeviceBuffer<uint32_t> W(n);
+  ScratchBuffer<uint32_t> W(n, s);
   ScratchBuffer<uint32_t> tmp(n, s), sval(2 * n, s);
   ScratchBuffer<TNode> tn(2 * n, s);
   ScratchBuffer<int32_t> lvl_a(n + 2, s), lvl_b(n + 2, s), ids(n + 2, s);
@@ -522,7 +522,7 @@ BinaryBvhHost build_tlas_gpu(const double* aabbs, size_t n, int max_leaf, int bi
     k_tlas_preorder<<<(unsigned)((levels[L].size() + 255) / 256), 256, 0, s>>>(tn.ptr, ids.ptr, (int)levels[L].size());
     VT_CUDA(cudaStreamSynchronize(s));
   }
-  DeviceBuffer<BinaryNode> nodes(total);
+  ScratchBuffer<BinaryNode> nodes(total, s);
   k_tlas_emit<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(tn.ptr, total, nmn.ptr, nmx.ptr, nodes.ptr);
   VT_CUDA(cudaGetLastError());
   BinaryBvhHost out;
