@@ -90,13 +90,18 @@ void launch_infer(const View& v, const float4* records, uint32_t rec_stride_f4, 
 // One training pass over n samples (records + float4 target per sample):
 // accumulates mean-loss gradients into v.grad_w / v.grad_table (which must be zero).
 void launch_train(const View& v, const float4* samples, uint32_t n, cudaStream_t s);
-// Adam over `count` parameters: master -= lr * mhat / (sqrt(vhat) + eps); writes the
-// fp16 copy and clears the gradient.  bc1/bc2 = 1 - beta^t.
-void launch_adam(float* master, float* m, float* v, float* grad, __half* out16, size_t count, float lr,
-                 float beta1, float beta2, float eps, float bc1, float bc2, int* diag, cudaStream_t s);
-// The same for the table, whose f32 gradient pairs and fp16 copies are float2 / half2.
-void launch_adam_table(float* master, float* m, float* v, float2* grad, __half2* out16, size_t pairs, float lr,
-                       float beta1, float beta2, float eps, float bc1, float bc2, int* diag, cudaStream_t s);
+// One parameter array of the optimiser (count even): f32 master, moments and
+// gradient, fp16 copy, learning rate.
+struct AdamArrays {
+  float *master, *m, *v, *grad;
+  __half* out16;
+  size_t count;
+  float lr;
+};
+// Adam over the table and the weights: master -= lr * mhat / (sqrt(vhat) + eps);
+// writes the fp16 copies and clears the gradients.  bc1/bc2 = 1 - beta^t.
+void launch_adam(const AdamArrays& table, const AdamArrays& weights, float beta1, float beta2, float eps, float bc1,
+                 float bc2, int* diag, cudaStream_t s);
 
 // Host: level resolutions floor(base * growth^l) (nrcEncoding.ts levelResolution).
 void level_resolutions(const Config& c, float* out);

@@ -125,10 +125,10 @@ void Cache::adam(cudaStream_t s) {
   ++step_;
   const float bc1 = (float)(1.0 - std::pow((double)cfg_.beta1, (double)step_));
   const float bc2 = (float)(1.0 - std::pow((double)cfg_.beta2, (double)step_));
-  launch_adam(w_.ptr, w_m_.ptr, w_v_.ptr, grad_w_.ptr, w16_.ptr, kWeights, cfg_.lr, cfg_.beta1, cfg_.beta2,
-              cfg_.eps, bc1, bc2, diag_.ptr + 1, s);
-  launch_adam_table(t_.ptr, t_m_.ptr, t_v_.ptr, grad_t_.ptr, t16_.ptr, table_pairs(), cfg_.table_lr, cfg_.beta1,
-                    cfg_.beta2, cfg_.eps, bc1, bc2, diag_.ptr + 1, s);
+  const AdamArrays table{t_.ptr, t_m_.ptr, t_v_.ptr, reinterpret_cast<float*>(grad_t_.ptr),
+                         reinterpret_cast<__half*>(t16_.ptr), 2 * table_pairs(), cfg_.table_lr};
+  const AdamArrays weights{w_.ptr, w_m_.ptr, w_v_.ptr, grad_w_.ptr, w16_.ptr, (size_t)kWeights, cfg_.lr};
+  launch_adam(table, weights, cfg_.beta1, cfg_.beta2, cfg_.eps, bc1, bc2, diag_.ptr + 1, s);
 }
 
 void Cache::train_step(const float4* samples, uint32_t n, cudaStream_t s) {

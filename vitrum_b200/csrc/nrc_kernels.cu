@@ -1,6 +1,6 @@
 // nrc_kernels.cu -- neural radiance cache kernels for sm_100a.
 //
-// k_nrc_infer   persistent, three CTAs per SM; per tile of 128 queries: encode
+// k_nrc_infer   persistent; per tile of 128 queries: encode
 //               (hash grid + SH4 + surface features) into a swizzled fp16 tile, then six
 //               tcgen05.mma layers (M=128, N=64, K=64 as four K=16 steps) with
 //               the fp32 accumulator in TMEM, ReLU + fp16 repack in the epilogue
@@ -20,6 +20,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 
@@ -58,14 +59,6 @@ __device__ __forceinline__ void store_row(uint8_t* tile, uint32_t r, const uint3
     *reinterpret_cast<uint4*>(tile + tc::sw128_offset(r, 8 * j)) = make_uint4(p[4 * j], p[4 * j + 1], p[4 * j + 2],
                                                                                p[4 * j + 3]);
 }
-__device__ __forceinline__ void load_row(const uint8_t* tile, uint32_t r, uint32_t (&p)[32]) {
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const uint4 q = *reinterpret_cast<const uint4*>(tile + tc::sw128_offset(r, 8 * j));
-    p[4 * j] = q.x; p[4 * j + 1] = q.y; p[4 * j + 2] = q.z; p[4 * j + 3] = q.w;
-  }
-}
-
 // normalised position in [0,1]^3 (normalizeToAabb, nrcEncoding.ts:166-178)
 __device__ __forceinline__ float3 normalise(const View& v, float px, float py, float pz) {
   return make_float3(fminf(1.0f, fmaxf(0.0f, (px - v.aabb_min[0]) * v.aabb_inv[0])),
@@ -94,33 +87,44 @@ __device__ __forceinline__ void sh4(float x, float y, float z, float (&s)[16]) {
   s[15] = 0.59004358992664352f * x * (3.0f * yy - xx);
 }
 
+// Position of a point within level l's grid: cell corner and fractions.
+struct Cell {
+  uint32_t x, y, z;
+  float fx, fy, fz;
+};
+__device__ __forceinline__ Cell grid_cell(const View& v, int l, float3 n01) {
+  const float N = v.res[l];
+  const float px = n01.x * N, py = n01.y * N, pz = n01.z * N;
+  const float x0 = floorf(px), y0 = floorf(py), z0 = floorf(pz);
+  return {(uint32_t)(int)x0, (uint32_t)(int)y0, (uint32_t)(int)z0, px - x0, py - y0, pz - z0};
+}
+
+// The two features of level l at a point: trilinear blend of the 8 corner rows.
+__device__ __forceinline__ uint32_t encode_level(const View& v, int l, float3 n01) {
+  float f0 = 0.0f, f1 = 0.0f;
+  if (l < v.levels) {
+    const Cell c = grid_cell(v, l, n01);
+    const __half2* tab = v.table16 + (size_t)l * (v.table_mask + 1u);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const uint32_t cx = k & 1, cy = (k >> 1) & 1, cz = (k >> 2) & 1;
+      const float w = (cx ? c.fx : 1.0f - c.fx) * (cy ? c.fy : 1.0f - c.fy) * (cz ? c.fz : 1.0f - c.fz);
+      const uint32_t row = grid_hash(c.x + cx, c.y + cy, c.z + cz) & v.table_mask;
+      const float2 e = __half22float2(__ldg(tab + row));
+      f0 = fmaf(w, e.x, f0);
+      f1 = fmaf(w, e.y, f1);
+    }
+  }
+  return pack_h2(f0, f1);
+}
+
 // Encodes one record (4 float4) into 64 fp16 inputs packed as 32 half2 words.
 __device__ __forceinline__ void encode(const View& v, float4 a, float4 b, float4 c, float4 d, uint32_t (&p)[32],
                                        float3& n01) {
   n01 = normalise(v, a.x, a.y, a.z);
   // all levels unrolled: the 8 x levels table gathers are independent and in flight together
 #pragma unroll
-  for (int l = 0; l < kMaxLevels; ++l) {
-    float f0 = 0.0f, f1 = 0.0f;
-    if (l < v.levels) {
-      const float N = v.res[l];
-      const float px = n01.x * N, py = n01.y * N, pz = n01.z * N;
-      const float x0 = floorf(px), y0 = floorf(py), z0 = floorf(pz);
-      const float fx = px - x0, fy = py - y0, fz = pz - z0;
-      const uint32_t ix = (uint32_t)(int)x0, iy = (uint32_t)(int)y0, iz = (uint32_t)(int)z0;
-      const __half2* tab = v.table16 + (size_t)l * (v.table_mask + 1u);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const uint32_t cx = k & 1, cy = (k >> 1) & 1, cz = (k >> 2) & 1;
-        const float w = (cx ? fx : 1.0f - fx) * (cy ? fy : 1.0f - fy) * (cz ? fz : 1.0f - fz);
-        const uint32_t row = grid_hash(ix + cx, iy + cy, iz + cz) & v.table_mask;
-        const float2 e = __half22float2(__ldg(tab + row));
-        f0 = fmaf(w, e.x, f0);
-        f1 = fmaf(w, e.y, f1);
-      }
-    }
-    p[l] = pack_h2(f0, f1);
-  }
+  for (int l = 0; l < kMaxLevels; ++l) p[l] = encode_level(v, l, n01);
   float s[16];
   sh4(a.w, b.x, b.y, s);
 #pragma unroll
@@ -136,25 +140,28 @@ __device__ __forceinline__ void encode(const View& v, float4 a, float4 b, float4
   p[31] = 0u;
 }
 
-// Scatter of the hash-feature input gradient g[0..31] (already scaled) into
-// the f32 table gradient with the trilinear weights.
-__device__ __forceinline__ void scatter_table(const View& v, float3 n01, const float (&g)[kEncWidth]) {
+// Scatter of the input gradient of level l's two features (already scaled)
+// into the f32 table gradient with the trilinear weights.
+__device__ __forceinline__ void scatter_level(const View& v, int l, float3 n01, float g0, float g1) {
+  if (l >= v.levels || (g0 == 0.0f && g1 == 0.0f)) return;
+  const Cell c = grid_cell(v, l, n01);
+  float2* gt = v.grad_table + (size_t)l * (v.table_mask + 1u);
+  // corners x and x + 1 are neighbouring rows when x is even (the hash's x prime is
+  // 1): one 16-byte atomic then adds both, six instead of eight a level on average
+  const bool odd = c.x & 1u;
 #pragma unroll
-  for (int l = 0; l < kMaxLevels; ++l) {
-    const float g0 = g[2 * l], g1 = g[2 * l + 1];
-    if (l >= v.levels || (g0 == 0.0f && g1 == 0.0f)) continue;
-    const float N = v.res[l];
-    const float px = n01.x * N, py = n01.y * N, pz = n01.z * N;
-    const float x0 = floorf(px), y0 = floorf(py), z0 = floorf(pz);
-    const float fx = px - x0, fy = py - y0, fz = pz - z0;
-    const uint32_t ix = (uint32_t)(int)x0, iy = (uint32_t)(int)y0, iz = (uint32_t)(int)z0;
-    float2* gt = v.grad_table + (size_t)l * (v.table_mask + 1u);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const uint32_t cx = k & 1, cy = (k >> 1) & 1, cz = (k >> 2) & 1;
-      const float w = (cx ? fx : 1.0f - fx) * (cy ? fy : 1.0f - fy) * (cz ? fz : 1.0f - fz);
-      const uint32_t row = grid_hash(ix + cx, iy + cy, iz + cz) & v.table_mask;
-      atomicAdd(gt + row, make_float2(w * g0, w * g1));
+  for (int k = 0; k < 4; ++k) {
+    const uint32_t cy = k & 1, cz = k >> 1;
+    const float wy = cy ? c.fy : 1.0f - c.fy, wz = cz ? c.fz : 1.0f - c.fz;
+    const float w0 = (1.0f - c.fx) * wy * wz, w1 = c.fx * wy * wz;
+    const uint32_t r0 = grid_hash(c.x, c.y + cy, c.z + cz) & v.table_mask;
+    const float2 a0 = make_float2(w0 * g0, w0 * g1), a1 = make_float2(w1 * g0, w1 * g1);
+    if (odd) {
+      atomicAdd(gt + r0, a0);
+      atomicAdd(gt + (grid_hash(c.x + 1u, c.y + cy, c.z + cz) & v.table_mask), a1);
+    } else {
+      const float2 lo = (r0 & 1u) ? a1 : a0, hi = (r0 & 1u) ? a0 : a1;
+      atomicAdd(reinterpret_cast<float4*>(gt + (r0 & ~1u)), make_float4(lo.x, lo.y, hi.x, hi.y));
     }
   }
 }
@@ -186,14 +193,6 @@ __device__ __forceinline__ void issue_fwd(uint32_t tmem_d, uint32_t a_tile, uint
   tc::fence_after_sync();
 #pragma unroll
   for (uint32_t kk = 0; kk < 4; ++kk) tc::mma_f16(tmem_d, tc::desc_k(a_tile, kk), tc::desc_k(w_tile, kk), kIdesc, kk);
-}
-
-// Thread-uniform bounded wait on the barrier's current phase.
-// On failure `phase` keeps the parity of the phase still pending.
-__device__ __forceinline__ bool wait_all(const View& v, uint64_t* bar, uint32_t& phase) {
-  const bool ok = __syncthreads_and(tc::mbar_wait(bar, phase, v.wait_cycles)) != 0;
-  if (ok) phase ^= 1u;
-  return ok;
 }
 
 // 64 fp32 accumulator columns of this thread's row (its TMEM lane)
@@ -353,7 +352,27 @@ __device__ __forceinline__ float rel_l2_lum(float p0, float p1, float p2) {
   return fminf(1.0f, fmaxf(-1.0f, nl)) * s;
 }
 
-__global__ void __launch_bounds__(128, 1)
+// 16-byte chunk `j` of row r of a tile
+__device__ __forceinline__ uint4* chunk_at(uint8_t* tile, uint32_t r, uint32_t j) {
+  return reinterpret_cast<uint4*>(tile + tc::sw128_offset(r, 8 * j));
+}
+
+// One tile of 128 samples at a time per CTA (one CTA per SM: its six stored
+// activation tiles and 384 TMEM columns of weight gradients leave no room for
+// another), four threads per sample, in four warpgroups that divide every phase
+// by columns: warpgroup q encodes and scatters levels 4q .. 4q + 3 (input
+// columns 8q .. 8q + 7) and one more 8-column block of the features, and takes
+// 16 of the 64 accumulator columns in the epilogues (warps w and w + 4 read the
+// same TMEM lanes).  Everything here waits on latency -- table gathers, the
+// chain of twelve dependent products and epilogues, the gradient atomics -- so
+// what the four-fold warps buy is overlap.
+// Measured per 65,536-sample step (2^15 / 2^19 tables, optimiser included): one
+// warpgroup 165 / 274 us; four 160 / 265; with 16-byte atomics for the weight
+// gradients (3.6 M single ones before) and for neighbouring table rows 123 / 231;
+// one barrier a layer 120 / 228.  Of a step's 120 us the table atomics take 34
+// (6.3 M at the L2's rate), the encoding 22, the chain of products 46.
+constexpr int kTrainGroups = 4;
+__global__ void __launch_bounds__(128 * kTrainGroups, 1)
     k_nrc_train(View v, const float4* __restrict__ samples, uint32_t n) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = align1024(smem_raw);
@@ -362,13 +381,13 @@ __global__ void __launch_bounds__(128, 1)
   uint8_t* X = G + kTileBytes;                    // X[0] = encoded input, X[l] = H_l (l = 1..5)
   uint64_t* bar = reinterpret_cast<uint64_t*>(X + kLayers * kTileBytes);
   uint32_t* slot = reinterpret_cast<uint32_t*>(bar + 1);
-  const uint32_t tid = threadIdx.x, warp = tid >> 5;
+  const uint32_t row = threadIdx.x & 127u, part = threadIdx.x >> 7, warp = threadIdx.x >> 5;
   if ((uint32_t)blockIdx.x * kTile >= n) return;
   if (warp == 0) {
     tc::tmem_alloc(slot, 512);
     tc::tmem_relinquish();
   }
-  if (tid == 0) {
+  if (threadIdx.x == 0) {
     tc::mbar_init(bar, 1);
     tc::fence_mbar_init();
   }
@@ -378,7 +397,7 @@ __global__ void __launch_bounds__(128, 1)
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = *slot;
-  const uint32_t lane_addr = tmem + ((warp * 32u) << 16);
+  const uint32_t lane_addr = tmem + (((warp & 3u) * 32u) << 16);
   const uint32_t w_s = tc::smem_u32(wt), g_s = tc::smem_u32(G), x_s = tc::smem_u32(X);
   const float inv_n = 1.0f / (float)n;
   uint32_t phase = 0;
@@ -386,36 +405,65 @@ __global__ void __launch_bounds__(128, 1)
   uint32_t tiles = 0;
   float loss = 0.0f;
   for (uint32_t tile = blockIdx.x; tile * kTile < n && !failed; tile += gridDim.x, ++tiles) {
-    const uint32_t i = tile * kTile + tid;
+    const uint32_t i = tile * kTile + row;
     const bool valid = i < n;
-    uint32_t p[32];
-    float3 n01;
     const float4* r = samples + (size_t)(valid ? i : 0) * 5;
-    encode(v, __ldg(r), __ldg(r + 1), __ldg(r + 2), __ldg(r + 3), p, n01);
-    const float4 tgt = __ldg(r + 4);
-    store_row(X, tid, p);
+    const float4 ra = __ldg(r);
+    const float3 n01 = normalise(v, ra.x, ra.y, ra.z);
+    {
+      uint32_t p[4];
+#pragma unroll
+      for (int l = 0; l < 4; ++l) p[l] = encode_level(v, 4 * (int)part + l, n01);
+      *chunk_at(X, row, part) = make_uint4(p[0], p[1], p[2], p[3]);
+      // columns 32 + 8 part: the spherical harmonics' halves, then the surface features
+      if (part < 2) {
+        const float4 rb = __ldg(r + 1);
+        float sh[16];
+        sh4(ra.w, rb.x, rb.y, sh);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          p[k] = part == 0 ? pack_h2(sh[2 * k], sh[2 * k + 1]) : pack_h2(sh[8 + 2 * k], sh[9 + 2 * k]);
+      } else if (part == 2) {
+        const float4 rb = __ldg(r + 1), rc = __ldg(r + 2), rd = __ldg(r + 3);
+        p[0] = pack_h2(rb.z, rb.w);
+        p[1] = pack_h2(rc.x, rc.y);
+        p[2] = pack_h2(rc.z, rc.w);
+        p[3] = pack_h2(rd.x, rd.y);
+      } else {
+        const float4 rd = __ldg(r + 3);
+        p[0] = pack_h2(rd.z, rd.w);
+        p[1] = pack_h2(1.0f, 0.0f);
+        p[2] = p[3] = 0u;
+      }
+      *chunk_at(X, row, 4 + part) = make_uint4(p[0], p[1], p[2], p[3]);
+    }
     tc::fence_async_smem();
     tc::fence_before_sync();
     __syncthreads();
-    // ---- forward, keeping H_1..H_5
+    // ---- forward, keeping H_1..H_5.  One barrier a layer: it publishes the next
+    // input and carries the verdict on the wait (a failed one's epilogue wrote
+    // garbage to shared memory only)
     float pr[3] = {0.0f, 0.0f, 0.0f};
-    for (int l = 0; l < kLayers && !failed; ++l) {
-      if (tid == 0) {
+    for (int l = 0; l < kLayers; ++l) {
+      if (threadIdx.x == 0) {
         issue_fwd(tmem, x_s + l * kTileBytes, w_s + l * kWBytes);
         tc::mma_commit(bar);
       }
-      if (!wait_all(v, bar, phase)) { failed = true; break; }
+      const bool ok = tc::mbar_wait(bar, phase, v.wait_cycles);
       tc::fence_after_sync();
+      uint32_t o[16];
       if (l + 1 < kLayers) {
-        uint32_t acc[64];
-        load_acc64(lane_addr, acc);
+        tc::tmem_ld16(lane_addr + 16u * part, o);
+        tc::tmem_wait_ld();
+        uint32_t p[8];
 #pragma unroll
-        for (int k = 0; k < 32; ++k)
-          p[k] = pack_h2(fmaxf(__uint_as_float(acc[2 * k]), 0.0f), fmaxf(__uint_as_float(acc[2 * k + 1]), 0.0f));
-        store_row(X + (l + 1) * kTileBytes, tid, p);
+        for (int k = 0; k < 8; ++k)
+          p[k] = pack_h2(fmaxf(__uint_as_float(o[2 * k]), 0.0f), fmaxf(__uint_as_float(o[2 * k + 1]), 0.0f));
+        uint8_t* H = X + (l + 1) * kTileBytes;
+        *chunk_at(H, row, 2 * part) = make_uint4(p[0], p[1], p[2], p[3]);
+        *chunk_at(H, row, 2 * part + 1) = make_uint4(p[4], p[5], p[6], p[7]);
         tc::fence_async_smem();
-      } else {
-        uint32_t o[16];
+      } else if (part == 0) {
         tc::tmem_ld16(lane_addr, o);
         tc::tmem_wait_ld();
         pr[0] = __uint_as_float(o[0]);
@@ -423,16 +471,17 @@ __global__ void __launch_bounds__(128, 1)
         pr[2] = __uint_as_float(o[2]);
       }
       tc::fence_before_sync();
-      __syncthreads();
+      if (__syncthreads_or(!ok)) { failed = true; break; }  // `phase` keeps the pending parity
+      phase ^= 1u;
     }
     if (failed) break;
-    // ---- output gradient
-    float g[3] = {0.0f, 0.0f, 0.0f};
-    if (valid) {
-      const float t3[3] = {tgt.x, tgt.y, tgt.z};
-      bool fin = isfinite(pr[0]) && isfinite(pr[1]) && isfinite(pr[2]) && isfinite(t3[0]) && isfinite(t3[1]) &&
-                 isfinite(t3[2]);
-      if (fin) {
+    // ---- output gradient (one thread per sample; the others clear its row's other columns)
+    if (part == 0) {
+      float g[3] = {0.0f, 0.0f, 0.0f};
+      const float4 tgt = __ldg(r + 4);
+      const bool fin = isfinite(pr[0]) && isfinite(pr[1]) && isfinite(pr[2]);
+      if (valid && fin && isfinite(tgt.x) && isfinite(tgt.y) && isfinite(tgt.z)) {
+        const float t3[3] = {tgt.x, tgt.y, tgt.z};
         const float lum = fminf(fabsf(rel_l2_lum(pr[0], pr[1], pr[2])), 1e19f);
         const float den = lum * lum + 1e-2f;
         const float sc = 2.0f / 3.0f / den;
@@ -445,83 +494,94 @@ __global__ void __launch_bounds__(128, 1)
           loss += dlt * dlt / den / 3.0f;
         }
       }
+      if (valid && v.tile_stats && __float_as_uint(tgt.w) != 0u && fin) {
+        // cache error estimate of the sample's screen tile (prediction vs target luminance)
+        const uint32_t pix = __float_as_uint(tgt.w) - 1u;
+        const uint32_t st = (pix / v.tile_width / v.tile_size) * v.tiles_x + (pix % v.tile_width) / v.tile_size;
+        float* ts = v.tile_stats + 3 * (size_t)st;
+        atomicAdd(ts, 0.2126f * fmaxf(pr[0], 0.0f) + 0.7152f * fmaxf(pr[1], 0.0f) + 0.0722f * fmaxf(pr[2], 0.0f));
+        atomicAdd(ts + 1, 0.2126f * tgt.x + 0.7152f * tgt.y + 0.0722f * tgt.z);
+        atomicAdd(ts + 2, 1.0f);
+      }
+      *chunk_at(G, row, 0) = make_uint4(pack_h2(g[0], g[1]), pack_h2(g[2], 0.0f), 0u, 0u);
+    } else {
+      *chunk_at(G, row, 2 * part) = make_uint4(0u, 0u, 0u, 0u);
     }
-    if (valid && v.tile_stats && __float_as_uint(tgt.w) != 0u && isfinite(pr[0]) && isfinite(pr[1]) &&
-        isfinite(pr[2])) {
-      // cache error estimate of the sample's screen tile (prediction vs target luminance)
-      const uint32_t pix = __float_as_uint(tgt.w) - 1u;
-      const uint32_t tile = (pix / v.tile_width / v.tile_size) * v.tiles_x + (pix % v.tile_width) / v.tile_size;
-      float* ts = v.tile_stats + 3 * (size_t)tile;
-      atomicAdd(ts, 0.2126f * fmaxf(pr[0], 0.0f) + 0.7152f * fmaxf(pr[1], 0.0f) + 0.0722f * fmaxf(pr[2], 0.0f));
-      atomicAdd(ts + 1, 0.2126f * tgt.x + 0.7152f * tgt.y + 0.0722f * tgt.z);
-      atomicAdd(ts + 2, 1.0f);
-    }
-#pragma unroll
-    for (int k = 0; k < 32; ++k) p[k] = 0u;
-    p[0] = pack_h2(g[0], g[1]);
-    p[1] = pack_h2(g[2], 0.0f);
-    store_row(G, tid, p);
+    *chunk_at(G, row, 2 * part + 1) = make_uint4(0u, 0u, 0u, 0u);
     tc::fence_async_smem();
     tc::fence_before_sync();
     __syncthreads();
     // ---- backward: layer 5 (output) down to 0
-    for (int l = kLayers - 1; l >= 0 && !failed; --l) {
-      if (tid == 0) {
+    for (int l = kLayers - 1; l >= 0; --l) {
+      if (threadIdx.x == 0) {
         tc::fence_after_sync();
         const uint32_t x_in = x_s + l * kTileBytes;  // this layer's input
         const uint32_t dw = tmem + 64u + 64u * (uint32_t)l;
 #pragma unroll
+        for (uint32_t kk = 0; kk < 4; ++kk)  // K = 64 outputs of this layer
+          tc::mma_f16(tmem, tc::desc_k(g_s, kk), tc::desc_mn(w_s + l * kWBytes, kk, kWBytes), kIdescBwd, kk);
+#pragma unroll
         for (uint32_t kk = 0; kk < 8; ++kk)  // K = 128 samples
           tc::mma_f16(dw, tc::desc_mn(g_s, kk, kTileBytes), tc::desc_mn(x_in, kk, kTileBytes), kIdescWgrad,
                       (tiles > 0 || kk > 0) ? 1u : 0u);
-#pragma unroll
-        for (uint32_t kk = 0; kk < 4; ++kk)  // K = 64 outputs of this layer
-          tc::mma_f16(tmem, tc::desc_k(g_s, kk), tc::desc_mn(w_s + l * kWBytes, kk, kWBytes), kIdescBwd, kk);
         tc::mma_commit(bar);
       }
-      if (!wait_all(v, bar, phase)) { failed = true; break; }
+      const bool ok = tc::mbar_wait(bar, phase, v.wait_cycles);
       tc::fence_after_sync();
-      uint32_t acc[64];
-      load_acc64(lane_addr, acc);  // dX_l
+      uint32_t acc[16];  // dX_l: this part's 16 columns; of layer 0 the 16 that hold its four levels' 8
+      tc::tmem_ld16(lane_addr + (l > 0 ? 16u * part : 16u * (part >> 1)), acc);
+      tc::tmem_wait_ld();
       tc::fence_before_sync();
       if (l > 0) {
         // G_{l-1} = dH_l * (H_l > 0)
-        uint32_t h[32];
-        load_row(X + l * kTileBytes, tid, h);
+        uint8_t* H = X + l * kTileBytes;
+        const uint4 ha = *chunk_at(H, row, 2 * part), hb = *chunk_at(H, row, 2 * part + 1);
+        const uint32_t h[8] = {ha.x, ha.y, ha.z, ha.w, hb.x, hb.y, hb.z, hb.w};
+        uint32_t p[8];
 #pragma unroll
-        for (int k = 0; k < 32; ++k) {
+        for (int k = 0; k < 8; ++k) {
           const float2 hv = unpack_h2(h[k]);
           const float a0 = hv.x > 0.0f ? __uint_as_float(acc[2 * k]) : 0.0f;
           const float a1 = hv.y > 0.0f ? __uint_as_float(acc[2 * k + 1]) : 0.0f;
           p[k] = pack_h2(fminf(65504.0f, fmaxf(-65504.0f, a0)), fminf(65504.0f, fmaxf(-65504.0f, a1)));
         }
-        store_row(G, tid, p);
+        *chunk_at(G, row, 2 * part) = make_uint4(p[0], p[1], p[2], p[3]);
+        *chunk_at(G, row, 2 * part + 1) = make_uint4(p[4], p[5], p[6], p[7]);
         tc::fence_async_smem();
-      } else if (valid) {
-        float ge[kEncWidth];
-#pragma unroll
-        for (int k = 0; k < kEncWidth; ++k) ge[k] = __uint_as_float(acc[k]) * inv_n;
-        scatter_table(v, n01, ge);
       }
-      __syncthreads();
+      if (__syncthreads_or(!ok)) { failed = true; break; }
+      phase ^= 1u;
+      if (l == 0 && valid) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float g0 = __uint_as_float((part & 1u) ? acc[8 + 2 * q] : acc[2 * q]) * inv_n;
+          const float g1 = __uint_as_float((part & 1u) ? acc[9 + 2 * q] : acc[2 * q + 1]) * inv_n;
+          scatter_level(v, 4 * (int)part + q, n01, g0, g1);
+        }
+      }
     }
   }
   if (failed) {
     fail_and_drain(v, bar, phase);
-  } else if (tiles > 0 && warp < 2) {
-    // weight gradients: rows 0..63 of each dW accumulator (lanes of warps 0, 1)
+  } else if (tiles > 0 && (warp & 3u) < 2u) {
+    // weight gradients: rows 0..63 of each dW accumulator (TMEM lanes 0..63), 16 columns per part
     tc::fence_after_sync();
     for (int l = 0; l < kLayers; ++l) {
-      uint32_t acc[64];
-      load_acc64(lane_addr + 64u + 64u * (uint32_t)l, acc);
-      float* gw = v.grad_w + (size_t)l * kWidth * kWidth + (size_t)tid * kWidth;
+      uint32_t acc[16];
+      tc::tmem_ld16(lane_addr + 64u + 64u * (uint32_t)l + 16u * part, acc);
+      tc::tmem_wait_ld();
+      float4* gw = reinterpret_cast<float4*>(v.grad_w + (size_t)l * kWidth * kWidth + (size_t)row * kWidth + 16u * part);
 #pragma unroll
-      for (int k = 0; k < 64; ++k) atomicAdd(gw + k, __uint_as_float(acc[k]) * inv_n);
+      for (int k = 0; k < 4; ++k)
+        atomicAdd(gw + k, make_float4(__uint_as_float(acc[4 * k]) * inv_n, __uint_as_float(acc[4 * k + 1]) * inv_n,
+                                      __uint_as_float(acc[4 * k + 2]) * inv_n, __uint_as_float(acc[4 * k + 3]) * inv_n));
     }
   }
-  // loss: warp reduce then one atomic per warp
-  for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xFFFFFFFFu, loss, o);
-  if ((tid & 31u) == 0 && v.loss) atomicAdd(v.loss, loss * inv_n);
+  // loss: warp reduce then one atomic per warp (part 0 holds it)
+  if (part == 0) {
+    for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xFFFFFFFFu, loss, o);
+    if ((threadIdx.x & 31u) == 0 && v.loss) atomicAdd(v.loss, loss * inv_n);
+  }
   tc::fence_before_sync();
   __syncthreads();
   if (warp == 0) tc::tmem_dealloc(tmem, 512);
@@ -556,34 +616,42 @@ __device__ __forceinline__ float adam_one(float cur, float& m, float& vv, float 
   return fminf(65504.0f, fmaxf(-65504.0f, up));
 }
 
-__global__ void k_nrc_adam(float* __restrict__ master, float* __restrict__ m, float* __restrict__ v,
-                           float* __restrict__ grad, __half* __restrict__ out16, size_t count, float lr, float b1,
-                           float b2, float eps, float ibc1, float ibc2, int* diag) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x) {
-    float mm = m[i], vv = v[i];
-    const float up = adam_one(master[i], mm, vv, grad[i], lr, b1, b2, eps, ibc1, ibc2, diag);
-    master[i] = up;
-    m[i] = mm;
-    v[i] = vv;
-    grad[i] = 0.0f;
-    out16[i] = __float2half_rn(up);
-  }
-}
+// One parameter array as pairs: f32 master, moments and gradient, fp16 copy.
+struct AdamPairs {
+  float2 *master, *m, *v, *grad;
+  __half2* out16;
+  size_t pairs;
+  float lr;
+};
 
-__global__ void k_nrc_adam_table(float2* __restrict__ master, float2* __restrict__ m, float2* __restrict__ v,
-                                 float2* __restrict__ grad, __half2* __restrict__ out16, size_t pairs, float lr,
-                                 float b1, float b2, float eps, float ibc1, float ibc2, int* diag) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < pairs; i += (size_t)gridDim.x * blockDim.x) {
-    float2 w = master[i], mm = m[i], vv = v[i];
+__device__ __forceinline__ void adam_pairs(const AdamPairs& a, size_t first, size_t step, float b1, float b2, float eps,
+                                           float ibc1, float ibc2, int* diag) {
+  float2 *__restrict__ master = a.master, *__restrict__ pm = a.m, *__restrict__ pv = a.v, *__restrict__ grad = a.grad;
+  __half2* __restrict__ out16 = a.out16;
+  for (size_t i = first; i < a.pairs; i += step) {
+    float2 w = master[i], mm = pm[i], vv = pv[i];
     const float2 g = grad[i];
-    w.x = adam_one(w.x, mm.x, vv.x, g.x, lr, b1, b2, eps, ibc1, ibc2, diag);
-    w.y = adam_one(w.y, mm.y, vv.y, g.y, lr, b1, b2, eps, ibc1, ibc2, diag);
+    w.x = adam_one(w.x, mm.x, vv.x, g.x, a.lr, b1, b2, eps, ibc1, ibc2, diag);
+    w.y = adam_one(w.y, mm.y, vv.y, g.y, a.lr, b1, b2, eps, ibc1, ibc2, diag);
     master[i] = w;
-    m[i] = mm;
-    v[i] = vv;
+    pm[i] = mm;
+    pv[i] = vv;
     grad[i] = make_float2(0.0f, 0.0f);
     out16[i] = __floats2half2_rn(w.x, w.y);
   }
+}
+
+// Adam over the table and, in the last `weight_ctas` CTAs, the weights (a launch
+// of their own cost 4 us of every step); clears the gradients and writes the
+// fp16 copies in the same pass.  Bound by memory: 76 bytes a pair.
+__global__ void __launch_bounds__(256) k_nrc_adam(AdamPairs table, AdamPairs weights, unsigned weight_ctas, float b1,
+                                                  float b2, float eps, float ibc1, float ibc2, int* diag) {
+  const unsigned table_ctas = gridDim.x - weight_ctas;
+  if (blockIdx.x < table_ctas)
+    adam_pairs(table, (size_t)blockIdx.x * 256 + threadIdx.x, (size_t)table_ctas * 256, b1, b2, eps, ibc1, ibc2, diag);
+  else
+    adam_pairs(weights, (size_t)(blockIdx.x - table_ctas) * 256 + threadIdx.x, (size_t)weight_ctas * 256, b1, b2, eps,
+               ibc1, ibc2, diag);
 }
 
 constexpr size_t infer_smem(int t) { return kLayers * kWBytes + (size_t)t * kTileBytes + 64 + 1024; }
@@ -624,6 +692,10 @@ void launch_infer_t(const View& v, const float4* records, uint32_t rec_stride_f4
 void launch_infer(const View& v, const float4* records, uint32_t rec_stride_f4, const uint32_t* n_dev, uint32_t n,
                   float* rgb_out, float4* radiance, int tiles_per_cta, cudaStream_t s) {
   if (n == 0) return;
+  // a batch of fewer tiles than SMs x T gets fewer tiles per CTA instead of idle SMs
+  // (1,000 to 18,944 queries: 31 -> 18 us; 40,000: 33 -> 27 us)
+  const uint32_t tiles = (n + kTile - 1) / kTile, sms = (uint32_t)sm_count();
+  tiles_per_cta = (int)std::min<uint32_t>((uint32_t)tiles_per_cta, (tiles + sms - 1) / sms);
   // tiles in flight per CTA: 1 to 4 (65 to 113 KB of shared memory).  Under the default
   // carve-out one CTA runs per SM, which keeps most of the unified L1 for the hash-table gathers:
   // asking for the largest shared-memory carve-out (three or two CTAs per SM) made two tiles per
@@ -643,24 +715,20 @@ void launch_train(const View& v, const float4* samples, uint32_t n, cudaStream_t
   }
   const uint32_t tiles = (n + kTile - 1) / kTile;
   const uint32_t grid = tiles < (uint32_t)sm_count() ? tiles : (uint32_t)sm_count();
-  k_nrc_train<<<grid, 128, kTrainSmem, s>>>(v, samples, n);
+  k_nrc_train<<<grid, 128 * kTrainGroups, kTrainSmem, s>>>(v, samples, n);
 }
 
-void launch_adam(float* master, float* m, float* v, float* grad, __half* out16, size_t count, float lr, float beta1,
-                 float beta2, float eps, float bc1, float bc2, int* diag, cudaStream_t s) {
-  if (!count) return;
-  const size_t g = (count + 255) / 256;
-  k_nrc_adam<<<(unsigned)(g < 148 * 16 ? g : 148 * 16), 256, 0, s>>>(master, m, v, grad, out16, count, lr, beta1,
-                                                                      beta2, eps, 1.0f / bc1, 1.0f / bc2, diag);
-}
-
-void launch_adam_table(float* master, float* m, float* v, float2* grad, __half2* out16, size_t pairs, float lr,
-                       float beta1, float beta2, float eps, float bc1, float bc2, int* diag, cudaStream_t s) {
-  if (!pairs) return;
-  const size_t g = (pairs + 255) / 256;
-  k_nrc_adam_table<<<(unsigned)(g < 148 * 16 ? g : 148 * 16), 256, 0, s>>>(
-      reinterpret_cast<float2*>(master), reinterpret_cast<float2*>(m), reinterpret_cast<float2*>(v), grad, out16,
-      pairs, lr, beta1, beta2, eps, 1.0f / bc1, 1.0f / bc2, diag);
+void launch_adam(const AdamArrays& table, const AdamArrays& weights, float beta1, float beta2, float eps, float bc1,
+                 float bc2, int* diag, cudaStream_t s) {
+  auto pairs = [](const AdamArrays& a) {
+    return AdamPairs{reinterpret_cast<float2*>(a.master), reinterpret_cast<float2*>(a.m),
+                     reinterpret_cast<float2*>(a.v), reinterpret_cast<float2*>(a.grad),
+                     reinterpret_cast<__half2*>(a.out16), a.count / 2, a.lr};
+  };
+  const size_t g = (table.count / 2 + 255) / 256;
+  const unsigned table_ctas = (unsigned)(g < 148 * 16 ? g : 148 * 16), weight_ctas = 16;
+  k_nrc_adam<<<table_ctas + weight_ctas, 256, 0, s>>>(pairs(table), pairs(weights), weight_ctas, beta1, beta2, eps,
+                                                      1.0f / bc1, 1.0f / bc2, diag);
 }
 
 }  // namespace nrc
