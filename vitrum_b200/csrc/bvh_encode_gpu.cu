@@ -8,12 +8,14 @@
 //      second child to arrive at a node (an atomic counter per node) computes
 //      its costs C(n), G(n, k) and splits from the children's, every value an
 //      IEEE-double operation in the host's order, ties to the first minimum;
-//   3. wide levels, top down, as the host's breadth-first queue: per level
-//      one thread per wide node picks its children (the plan's frontier or the
-//      reference's greedy rule) and slots; an exclusive scan over the level
-//      gives each node its child base and record block, so numbering equals
-//      the host's queue order; each node's 80 bytes and its leaf records are
-//      then written, the internal children listed for the next level.
+//   3. wide levels, top down, as the host's breadth-first queue, eight lanes per
+//      wide node: per level the node's children (the plan's frontier or the
+//      reference's greedy rule) are picked and put into slots (lane i holds child
+//      i); an exclusive scan over the level gives each node its child base and
+//      record block, so numbering equals the host's queue order; then lane s
+//      quantises slot s, writes its records or lists its child for the next level.
+//      The levels follow one another on the stream; the host reads their sizes
+//      once per batch.
 // Quantised child bounds are rounded outward exactly: each grid corner
 // origin + q * 2^e is compared with the child bound through a nonoverlapping
 // expansion of the sum (Shewchuk's grow-expansion of TwoSums), whose largest
@@ -185,105 +187,145 @@ __device__ __forceinline__ int greedy_children(const BinaryNode* nodes, uint32_t
   return n;
 }
 
-// Greedy slot assignment (the host's assign_slots), IEEE doubles in its order.
-// Each (child, slot) cost is recomputed where it is compared (the same
-// operations, so the same value) instead of being kept in an 8 x 8 array, and
-// the slots come back packed in registers: slot of child i in bits 4i..4i+3.
-__device__ __forceinline__ uint32_t assign_slots(const BinaryNode* nodes, const BinaryNode& parent, const uint32_t* ch,
-                                                 int n) {
-  const double pcx = __dmul_rn(0.5, __dadd_rn((double)parent.mn[0], (double)parent.mx[0]));
-  const double pcy = __dmul_rn(0.5, __dadd_rn((double)parent.mn[1], (double)parent.mx[1]));
-  const double pcz = __dmul_rn(0.5, __dadd_rn((double)parent.mn[2], (double)parent.mx[2]));
-  double dx[8], dy[8], dz[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    if (i >= n) { dx[i] = dy[i] = dz[i] = 0.0; continue; }
-    const BinaryNode c = nodes[ch[i] & ~kMerged];
-    dx[i] = __dsub_rn(__dmul_rn(0.5, __dadd_rn((double)c.mn[0], (double)c.mx[0])), pcx);
-    dy[i] = __dsub_rn(__dmul_rn(0.5, __dadd_rn((double)c.mn[1], (double)c.mx[1])), pcy);
-    dz[i] = __dsub_rn(__dmul_rn(0.5, __dadd_rn((double)c.mn[2], (double)c.mx[2])), pcz);
+// Greedy slot assignment (the host's assign_slots), IEEE doubles in its order,
+// by the eight lanes of a node's group: lane i holds child i (i < n) and finds
+// its cheapest free slot, the group takes the cheapest (child, slot) of all, ties
+// to the lower child and slot.  Returns the slot of child i in lane i.
+__device__ __forceinline__ int assign_slots(const BinaryNode* nodes, const BinaryNode& parent, uint32_t ch, int n) {
+  const int i = (int)(threadIdx.x & 7u);
+  double dx = 0.0, dy = 0.0, dz = 0.0;
+  if (i < n) {
+    const BinaryNode c = nodes[ch & ~kMerged];
+    const double pcx = __dmul_rn(0.5, __dadd_rn((double)parent.mn[0], (double)parent.mx[0]));
+    const double pcy = __dmul_rn(0.5, __dadd_rn((double)parent.mn[1], (double)parent.mx[1]));
+    const double pcz = __dmul_rn(0.5, __dadd_rn((double)parent.mn[2], (double)parent.mx[2]));
+    dx = __dsub_rn(__dmul_rn(0.5, __dadd_rn((double)c.mn[0], (double)c.mx[0])), pcx);
+    dy = __dsub_rn(__dmul_rn(0.5, __dadd_rn((double)c.mn[1], (double)c.mx[1])), pcy);
+    dz = __dsub_rn(__dmul_rn(0.5, __dadd_rn((double)c.mn[2], (double)c.mx[2])), pcz);
   }
-  uint32_t used_c = 0, used_s = 0, slots = 0xFFFFFFFFu;
-  for (int round = 0; round < n; ++round) {
-    int bi = -1, bs = -1;
+  uint32_t used = 0;
+  int slot = -1;
+  const int rounds = (int)__reduce_max_sync(0xFFFFFFFFu, (unsigned)n);  // the warp's four groups go together
+  for (int round = 0; round < rounds; ++round) {
     double bc = INFINITY;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      if (i >= n || ((used_c >> i) & 1u)) continue;
+    int at = 64;  // 8 * child + slot; 64: nothing to offer
+    if (i < n && slot < 0) {
 #pragma unroll
       for (int s = 0; s < 8; ++s) {
-        if ((used_s >> s) & 1u) continue;
+        if ((used >> s) & 1u) continue;
         const double sx = (s & 4) ? -1.0 : 1.0, sy = (s & 2) ? -1.0 : 1.0, sz = (s & 1) ? -1.0 : 1.0;
-        const double cost = __dadd_rn(__dadd_rn(__dmul_rn(dx[i], sx), __dmul_rn(dy[i], sy)), __dmul_rn(dz[i], sz));
-        if (bi < 0 || cost < bc) { bc = cost; bi = i; bs = s; }
+        const double cost = __dadd_rn(__dadd_rn(__dmul_rn(dx, sx), __dmul_rn(dy, sy)), __dmul_rn(dz, sz));
+        if (at == 64 || cost < bc) { bc = cost; at = 8 * i + s; }
       }
     }
-    used_c |= 1u << bi;
-    used_s |= 1u << bs;
-    slots = (slots & ~(0xFu << (4 * bi))) | ((uint32_t)bs << (4 * bi));
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+      const double oc = __shfl_xor_sync(0xFFFFFFFFu, bc, o);
+      const int oa = __shfl_xor_sync(0xFFFFFFFFu, at, o);
+      if (oa != 64 && (at == 64 || oc < bc || (oc == bc && oa < at))) { bc = oc; at = oa; }
+    }
+    if (at != 64) {
+      used |= 1u << (at & 7);
+      if ((at >> 3) == i) slot = at & 7;
+    }
   }
-  return slots;
+  return slot;
 }
-
-struct LevelPlan {
-  uint32_t ch[8];      // children (binary ids; kMerged: a subtree's leaf slot)
-  int8_t slot_of[8];
-  int32_t n;
-};
 
 // is child entry e a leaf slot?  (a merged subtree, or a binary leaf)
 __device__ __forceinline__ bool entry_is_leaf(const BinaryNode* nodes, uint32_t e) {
   return (e & kMerged) || leaf_word(nodes[e].w7);
 }
 
+// A level of wide nodes: its node count, first node and first record; entry L + 1
+// is written by level L's scan.
+struct LevelState {
+  uint32_t n, start, rec;
+};
+constexpr int kMaxLevels = 64;  // the binary tree is at most 58 deep
+struct EncodeState {
+  LevelState level[kMaxLevels + 1];
+  uint32_t stop;   // level + 1 that ran out of records (its emission waits for a larger array); ~0: too many nodes
+  uint32_t err;    // records beyond 2^30
+};
+// Device arrays of one encoding.
+struct EncodeWork {
+  EncodeState* state;
+  uint32_t* list[2];   // binary nodes of a level's wide nodes, by level parity
+  uint32_t* slots;     // per node of the level: the child entry of each slot (kNone: empty)
+  uint32_t* n_int;     // per node: internal children, then their offset
+  uint32_t* span;      // per node: records, then their offset
+  uint32_t max_wide;
+};
+constexpr int kEncodeThreads = 128;
+constexpr int kEncodeNodes = kEncodeThreads / 8;
+
 // sah: 0 the reference's greedy collapse, else the SAH-optimal collapse at that width (2..8)
-__global__ void k_level_plan(const BinaryNode* __restrict__ nodes, const DpNode* __restrict__ dp, int sah,
-                             const uint32_t* __restrict__ level, uint32_t n_level, LevelPlan* __restrict__ plan,
-                             uint32_t* __restrict__ n_int, uint32_t* __restrict__ span) {
-  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n_level) return;
-  const uint32_t x = level[j];
-  LevelPlan p;
-  int n;
-  if (sah) {
-    n = 0;
-    if (leaf_word(nodes[x].w7)) {
-      p.ch[0] = x;
-      n = 1;
-    } else {
-      const int s = dp[x].split[sah - 2];
-      frontier(nodes, dp, x + 1, s, p.ch, n);
-      frontier(nodes, dp, x + nodes[x].w6, sah - s, p.ch, n);
+__global__ void __launch_bounds__(kEncodeThreads) k_level_plan(const BinaryNode* __restrict__ nodes,
+                                                               const DpNode* __restrict__ dp, int sah, EncodeWork w,
+                                                               int level) {
+  constexpr uint32_t kAll = 0xFFFFFFFFu;
+  if (w.state->stop) return;
+  const uint32_t n_level = w.state->level[level].n;
+  const int i = (int)(threadIdx.x & 7u), shift = (int)(threadIdx.x & 24u);
+  __shared__ uint32_t pick[kEncodeNodes][8];
+  uint32_t* mine = pick[threadIdx.x >> 3];
+  for (uint32_t base = blockIdx.x * kEncodeNodes; base < n_level; base += gridDim.x * kEncodeNodes) {
+    const uint32_t j = base + (threadIdx.x >> 3);
+    const bool on = j < n_level;
+    const uint32_t x = on ? w.list[level & 1][j] : 0u;
+    int n = 0;
+    if (on && i == 0) {
+      if (sah) {
+        if (leaf_word(nodes[x].w7)) {
+          mine[0] = x;
+          n = 1;
+        } else {
+          const int s = dp[x].split[sah - 2];
+          frontier(nodes, dp, x + 1, s, mine, n);
+          frontier(nodes, dp, x + nodes[x].w6, sah - s, mine, n);
+        }
+      } else {
+        n = greedy_children(nodes, x, mine);
+      }
     }
-  } else {
-    n = greedy_children(nodes, x, p.ch);
-  }
-  const uint32_t slots = assign_slots(nodes, nodes[x], p.ch, n);
-  uint32_t internal = 0;
-  int first_leaf = 8, last_leaf = -1;
-  for (int i = 0; i < n; ++i) {
-    const int si = (int)((slots >> (4 * i)) & 0xFu);
-    p.slot_of[i] = (int8_t)si;
-    if (entry_is_leaf(nodes, p.ch[i])) {
-      first_leaf = min(first_leaf, si);
-      last_leaf = max(last_leaf, si);
-    } else {
-      ++internal;
+    __syncwarp();
+    n = __shfl_sync(kAll, n, shift);
+    const uint32_t ch = i < n ? mine[i] : kNone;
+    const int slot = assign_slots(nodes, nodes[x], ch, n);
+    const bool leaf = i < n && entry_is_leaf(nodes, ch);
+    // the masks by slot: lane i speaks for slot `slot`
+    uint32_t at = i < n ? 1u << slot : 0u, leaves = leaf ? at : 0u;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+      at |= __shfl_xor_sync(kAll, at, o);
+      leaves |= __shfl_xor_sync(kAll, leaves, o);
     }
+    if (on) {
+      uint32_t* out = w.slots + 8 * (size_t)j;
+      if (i < n) out[slot] = ch;
+      if (!((at >> i) & 1u)) out[i] = kNone;
+      if (i == 0) {
+        w.n_int[j] = (uint32_t)__popc(at & ~leaves);
+        w.span[j] = leaves ? 4u * (uint32_t)((31 - __clz(leaves)) - (__ffs(leaves) - 1)) + 4u : 0u;
+      }
+    }
+    __syncwarp();
   }
-  for (int i = n; i < 8; ++i) p.slot_of[i] = -1;
-  p.n = n;
-  plan[j] = p;
-  n_int[j] = internal;
-  span[j] = last_leaf >= 0 ? (uint32_t)(4 * (last_leaf - first_leaf) + 4) : 0u;
 }
 
-// Exclusive scans of two arrays in one CTA (levels are at most a few 100 k nodes).
-__global__ void k_scan2(uint32_t* __restrict__ a, uint32_t* __restrict__ b, uint32_t n,
-                        unsigned long long* __restrict__ totals) {
+// Exclusive scans of a level's two counts in one CTA (levels are at most a few
+// 100 k nodes), and the next level's state.
+__global__ void __launch_bounds__(1024) k_level_scan(EncodeWork w, int level, uint32_t rec_cap) {
   __shared__ unsigned long long wa[32], wb[32];
   __shared__ unsigned long long carry_a, carry_b;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  EncodeState* st = w.state;
+  if (st->stop) return;
+  uint32_t* a = w.n_int;
+  uint32_t* b = w.span;
+  const LevelState cur = st->level[level];
+  const uint32_t n = cur.n;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (threadIdx.x == 0) { carry_a = 0; carry_b = 0; }
   __syncthreads();
   for (uint32_t base = 0; base < n; base += blockDim.x) {
@@ -294,7 +336,7 @@ __global__ void k_scan2(uint32_t* __restrict__ a, uint32_t* __restrict__ b, uint
       const unsigned long long ta = __shfl_up_sync(0xFFFFFFFFu, sa, o), tb = __shfl_up_sync(0xFFFFFFFFu, sb, o);
       if (lane >= o) { sa += ta; sb += tb; }
     }
-    if (lane == 31) { wa[w] = sa; wb[w] = sb; }
+    if (lane == 31) { wa[wid] = sa; wb[wid] = sb; }
     __syncthreads();
     if (threadIdx.x == 0) {
       unsigned long long ra = carry_a, rb = carry_b;
@@ -310,14 +352,15 @@ __global__ void k_scan2(uint32_t* __restrict__ a, uint32_t* __restrict__ b, uint
     }
     __syncthreads();
     if (i < n) {
-      a[i] = (uint32_t)(wa[w] + sa - va);
-      b[i] = (uint32_t)(wb[w] + sb - vb);
+      a[i] = (uint32_t)(wa[wid] + sa - va);
+      b[i] = (uint32_t)(wb[wid] + sb - vb);
     }
     __syncthreads();
   }
   if (threadIdx.x == 0) {
-    totals[0] = carry_a;
-    totals[1] = carry_b;
+    st->level[level + 1] = {(uint32_t)carry_a, cur.start + cur.n, (uint32_t)(cur.rec + carry_b)};
+    if (cur.start + cur.n + carry_a > w.max_wide) st->stop = ~0u;
+    else if (cur.rec + carry_b > rec_cap) st->stop = (uint32_t)level + 1u;
   }
 }
 
@@ -370,108 +413,104 @@ struct EmitArgs {
   uint32_t node_base, rec_base;
 };
 
-__global__ void k_level_emit(EmitArgs A, const uint32_t* __restrict__ level, uint32_t n_level,
-                             const LevelPlan* __restrict__ plan, const uint32_t* __restrict__ int_off,
-                             const uint32_t* __restrict__ rec_off, uint32_t level_start, uint32_t rec_start,
-                             uint32_t* __restrict__ words, float* __restrict__ recs, uint32_t* __restrict__ next,
-                             int* __restrict__ err) {
-  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n_level) return;
-  const BinaryNode parent = A.nodes[level[j]];
-  const LevelPlan p = plan[j];
-  int child_at_slot[8];
-  for (int s = 0; s < 8; ++s) child_at_slot[s] = -1;
-  for (int i = 0; i < p.n; ++i) child_at_slot[p.slot_of[i]] = i;
-  uint32_t wl[20];
-  for (int k = 0; k < 20; ++k) wl[k] = 0;
-  uint8_t* bytes = reinterpret_cast<uint8_t*>(wl);
-  const float pm[3] = {parent.mn[0], parent.mn[1], parent.mn[2]};
-  memcpy(bytes, pm, 12);
-  int ex[3];
-  for (int k = 0; k < 3; ++k) {
-    ex[k] = grid_exponent(parent.mn[k], parent.mx[k]);
-    bytes[12 + k] = (uint8_t)(ex[k] + 127);
+// The record of triangle (or instance) src.
+__device__ __forceinline__ void write_record(const EmitArgs& A, uint32_t src, float4* rec) {
+  if (A.inst_recs) {
+    const float4* in = reinterpret_cast<const float4*>(A.inst_recs) + 4 * (size_t)src;
+    for (int k = 0; k < 4; ++k) rec[k] = in[k];
+    return;
   }
-  uint8_t imask = 0;
-  const uint32_t child_base = A.node_base + level_start + n_level + int_off[j];
-  int first_leaf = 8;
-  for (int s = 0; s < 8; ++s) {
-    const int ci = child_at_slot[s];
-    if (ci >= 0 && entry_is_leaf(A.nodes, p.ch[ci])) { first_leaf = s; break; }
-  }
-  const uint32_t block = rec_start + rec_off[j];
-  const uint32_t tri_base = A.rec_base + block - 4u * (uint32_t)(first_leaf < 8 ? first_leaf : 0);
-  if ((unsigned long long)A.rec_base + block + 32 >= 0x40000000ull) atomicOr(err, 1);
-  uint32_t tri_valid = 0;
-  uint32_t q_int = 0;
-  uint8_t* qlo = bytes + 32;
-  uint8_t* qhi = bytes + 56;
-  for (int s = 0; s < 8; ++s) {
-    const int ci = child_at_slot[s];
-    if (ci < 0) {
-      for (int k = 0; k < 3; ++k) { qlo[k * 8 + s] = 255; qhi[k * 8 + s] = 0; }
-      continue;
-    }
-    const uint32_t e = p.ch[ci];
-    const uint32_t id = e & ~kMerged;
-    const BinaryNode c = A.nodes[id];
-    for (int k = 0; k < 3; ++k) {
-      const double step = ldexp(1.0, ex[k]);
-      const double lo = floor(__ddiv_rn(__dsub_rn((double)c.mn[k], (double)pm[k]), step));
-      const double hi = ceil(__ddiv_rn(__dsub_rn((double)c.mx[k], (double)pm[k]), step));
-      int ql = (int)fmin(255.0, fmax(0.0, lo));
-      int qh = (int)fmin(255.0, fmax(0.0, hi));
-      while (ql > 0 && corner_sign(pm[k], ql, ex[k], c.mn[k]) > 0) --ql;
-      while (qh < 255 && corner_sign(pm[k], qh, ex[k], c.mx[k]) < 0) ++qh;
-      qlo[k * 8 + s] = (uint8_t)ql;
-      qhi[k * 8 + s] = (uint8_t)qh;
-    }
-    if (entry_is_leaf(A.nodes, e)) {
-      uint32_t first, cnt;
-      if (e & kMerged) {
-        first = A.dp[id].first;
-        cnt = A.dp[id].count;
+  const uint32_t* iv = A.idx + (size_t)src * A.is;
+  float v[3][3];
+  for (int vi = 0; vi < 3; ++vi)
+    for (int k = 0; k < 3; ++k) v[vi][k] = A.pos[(size_t)iv[vi] * A.ps + k];
+  const uint32_t mat = A.tri_mat ? A.tri_mat[src] : 0u;
+  float nn[3] = {0, 0, 0};
+  const bool valid = reference_normal(v[0], v[1], v[2], nn);
+  const uint32_t flags = valid && A.mat_flags && A.tri_mat ? A.mat_flags[mat] : 0u;
+  rec[0] = make_float4(v[0][0], v[0][1], v[0][2], __uint_as_float(src));
+  rec[1] = make_float4(v[1][0], v[1][1], v[1][2], A.tri_mat ? __uint_as_float(mat) : 0.0f);
+  rec[2] = make_float4(v[2][0], v[2][1], v[2][2], __uint_as_float(flags));
+  rec[3] = make_float4(nn[0], nn[1], nn[2], valid ? 1.0f : 0.0f);
+}
+
+__global__ void __launch_bounds__(kEncodeThreads) k_level_emit(EmitArgs A, EncodeWork w, int level,
+                                                               uint32_t* __restrict__ words, float* __restrict__ recs) {
+  constexpr uint32_t kAll = 0xFFFFFFFFu;
+  if (w.state->stop) return;
+  const LevelState st = w.state->level[level];
+  const int s = (int)(threadIdx.x & 7u), shift = (int)(threadIdx.x & 24u);
+  uint32_t* next = w.list[(level & 1) ^ 1];
+  for (uint32_t base = blockIdx.x * kEncodeNodes; base < st.n; base += gridDim.x * kEncodeNodes) {
+    const uint32_t j = base + (threadIdx.x >> 3);
+    const bool on = j < st.n;
+    const uint32_t e = on ? w.slots[8 * (size_t)j + s] : kNone;
+    const bool child = e != kNone, leaf = child && entry_is_leaf(A.nodes, e);
+    const uint32_t all = (__ballot_sync(kAll, child) >> shift) & 0xFFu;
+    const uint32_t leaves = (__ballot_sync(kAll, leaf) >> shift) & 0xFFu, imask = all & ~leaves;
+    const BinaryNode parent = A.nodes[on ? w.list[level & 1][j] : 0u];
+    const float pm[3] = {parent.mn[0], parent.mn[1], parent.mn[2]};
+    int mine = 0;  // lane k < 3: axis k's grid exponent
+    if (s < 3) mine = grid_exponent(s == 0 ? pm[0] : (s == 1 ? pm[1] : pm[2]),
+                                    s == 0 ? parent.mx[0] : (s == 1 ? parent.mx[1] : parent.mx[2]));
+    int ex[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) ex[k] = __shfl_sync(kAll, mine, shift + k);
+    const uint32_t first_leaf = leaves ? (uint32_t)(__ffs(leaves) - 1) : 0u;
+    const uint32_t int_off = on ? w.n_int[j] : 0u, block = st.rec + (on ? w.span[j] : 0u);
+    uint32_t* out = words + 20 * (size_t)(st.start + j);
+    uint32_t valid = 0;
+    if (on) {
+      uint8_t* bytes = reinterpret_cast<uint8_t*>(out);
+      uint8_t* qlo = bytes + 32 + s;
+      uint8_t* qhi = bytes + 56 + s;
+      if (!child) {
+        for (int k = 0; k < 3; ++k) { qlo[8 * k] = 255; qhi[8 * k] = 0; }
       } else {
-        first = c.w6;
-        cnt = c.w7 & 0xFFFFu;
-      }
-      tri_valid |= ((1u << cnt) - 1u) << (4 * s);
-      float* out = recs + 16 * ((size_t)block + 4 * (s - first_leaf));
-      for (uint32_t t = 0; t < cnt; ++t) {
-        const uint32_t src = A.order[first + t];
-        float* rec = out + 16 * t;
-        if (A.inst_recs) {
-          for (int k = 0; k < 16; ++k) rec[k] = A.inst_recs[16 * (size_t)src + k];
-          continue;
+        const uint32_t id = e & ~kMerged;
+        const BinaryNode c = A.nodes[id];
+        for (int k = 0; k < 3; ++k) {
+          const double step = ldexp(1.0, ex[k]);
+          const double lo = floor(__ddiv_rn(__dsub_rn((double)c.mn[k], (double)pm[k]), step));
+          const double hi = ceil(__ddiv_rn(__dsub_rn((double)c.mx[k], (double)pm[k]), step));
+          int ql = (int)fmin(255.0, fmax(0.0, lo));
+          int qh = (int)fmin(255.0, fmax(0.0, hi));
+          while (ql > 0 && corner_sign(pm[k], ql, ex[k], c.mn[k]) > 0) --ql;
+          while (qh < 255 && corner_sign(pm[k], qh, ex[k], c.mx[k]) < 0) ++qh;
+          qlo[8 * k] = (uint8_t)ql;
+          qhi[8 * k] = (uint8_t)qh;
         }
-        const uint32_t* iv = A.idx + (size_t)src * A.is;
-        float v[3][3];
-        for (int vi = 0; vi < 3; ++vi)
-          for (int k = 0; k < 3; ++k) v[vi][k] = A.pos[(size_t)iv[vi] * A.ps + k];
-        for (int vi = 0; vi < 3; ++vi)
-          for (int k = 0; k < 3; ++k) rec[4 * vi + k] = v[vi][k];
-        rec[3] = __uint_as_float(src);
-        rec[7] = A.tri_mat ? __uint_as_float(A.tri_mat[src]) : 0.0f;
-        rec[11] = 0.0f;
-        float nn[3] = {0, 0, 0};
-        const bool valid = reference_normal(v[0], v[1], v[2], nn);
-        rec[12] = nn[0];
-        rec[13] = nn[1];
-        rec[14] = nn[2];
-        rec[15] = valid ? 1.0f : 0.0f;
-        if (valid && A.mat_flags && A.tri_mat) rec[11] = __uint_as_float(A.mat_flags[A.tri_mat[src]]);
+        if (leaf) {
+          uint32_t first, cnt;
+          if (e & kMerged) {
+            first = A.dp[id].first;
+            cnt = A.dp[id].count;
+          } else {
+            first = c.w6;
+            cnt = c.w7 & 0xFFFFu;
+          }
+          valid = ((1u << cnt) - 1u) << (4 * s);
+          float* to = recs + 16 * ((size_t)block + 4 * (s - first_leaf));
+          for (uint32_t t = 0; t < cnt; ++t) write_record(A, A.order[first + t], reinterpret_cast<float4*>(to + 16 * t));
+        } else {
+          next[int_off + (uint32_t)__popc(imask & ((1u << s) - 1u))] = id;
+        }
       }
-    } else {
-      imask |= (uint8_t)(1u << s);
-      next[int_off[j] + q_int++] = id;
+    }
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) valid |= __shfl_xor_sync(kAll, valid, o);
+    if (on && s == 0) {
+      if ((unsigned long long)A.rec_base + block + 32 >= 0x40000000ull) atomicOr(&w.state->err, 1u);
+      out[0] = __float_as_uint(pm[0]);
+      out[1] = __float_as_uint(pm[1]);
+      out[2] = __float_as_uint(pm[2]);
+      out[3] = (uint32_t)(ex[0] + 127) | (uint32_t)(ex[1] + 127) << 8 | (uint32_t)(ex[2] + 127) << 16 | imask << 24;
+      out[4] = A.node_base + st.start + st.n + int_off;
+      out[5] = A.rec_base + block - 4u * first_leaf;
+      out[6] = valid;
+      out[7] = 0u;
     }
   }
-  memcpy(bytes + 24, &tri_valid, 4);
-  bytes[15] = imask;
-  memcpy(bytes + 16, &child_base, 4);
-  memcpy(bytes + 20, &tri_base, 4);
-  uint32_t* w = words + 20 * (size_t)(level_start + j);
-  for (int k = 0; k < 20; ++k) w[k] = wl[k];
 }
 
 }  // namespace
@@ -520,51 +559,58 @@ WideBvhHost encode_wide_gpu(const BinaryBvhDevice& bin, const float* d_pos, int 
   size_t rec_cap = 28 + 4 * (size_t)bin.ntri + 64;
   ScratchBuffer<float> recs(16 * rec_cap, s);
   VT_CUDA(cudaMemsetAsync(recs.ptr, 0, recs.bytes(), s));
-  ScratchBuffer<uint32_t> lvl_a(max_wide, s), lvl_b(max_wide, s), n_int(max_wide, s), span(max_wide, s);
-  ScratchBuffer<LevelPlan> plan(max_wide, s);
-  ScratchBuffer<unsigned long long> totals(2, s);
-  ScratchBuffer<int> err(1, s);
-  VT_CUDA(cudaMemsetAsync(err.ptr, 0, sizeof(int), s));
-  const uint32_t root = 0;
-  VT_CUDA(cudaMemcpyAsync(lvl_a.ptr, &root, sizeof root, cudaMemcpyHostToDevice, s));
+  ScratchBuffer<uint32_t> lvl_a(max_wide, s), lvl_b(max_wide, s), n_int(max_wide, s), span(max_wide, s),
+      slots(8 * (size_t)max_wide, s);
+  ScratchBuffer<EncodeState> state(1, s);
+  EncodeWork w{state.ptr, {lvl_a.ptr, lvl_b.ptr}, slots.ptr, n_int.ptr, span.ptr, max_wide};
+  EncodeState st{};
+  st.level[0] = {1u, 0u, 28u};
+  VT_CUDA(cudaMemcpyAsync(state.ptr, &st, sizeof st, cudaMemcpyHostToDevice, s));
+  VT_CUDA(cudaMemsetAsync(lvl_a.ptr, 0, sizeof(uint32_t), s));  // the root
   EmitArgs A{bin.nodes.ptr, sah ? dp.ptr : nullptr, bin.order.ptr, d_pos, pos_stride, d_idx, idx_stride, d_tri_mat,
              d_mat_flags, d_inst_recs, node_base, rec_base};
-  uint32_t level_n = 1, level_start = 0, rec_used = 28;
+  // A level holds at most eight times the one above; levels beyond the last are empty
+  // launches.  The first batch covers a tree of four children per wide node.
+  auto blocks = [&](int level) {
+    const uint32_t most = level < 8 ? (uint32_t)std::min<uint64_t>(1ull << (3 * level), max_wide) : max_wide;
+    return std::min<unsigned>((most + kEncodeNodes - 1) / kEncodeNodes, 148 * 16);
+  };
+  int level = 0, batch = 2;
+  for (uint32_t q = max_wide; q > 1; q >>= 2) ++batch;
   int depth = 0;
-  ScratchBuffer<uint32_t>* cur = &lvl_a;
-  ScratchBuffer<uint32_t>* nxt = &lvl_b;
-  while (level_n) {
-    ++depth;
-    const unsigned blocks = (level_n + 127) / 128;
-    k_level_plan<<<blocks, 128, 0, s>>>(bin.nodes.ptr, sah ? dp.ptr : nullptr, sah ? width : 0, cur->ptr, level_n,
-                                        plan.ptr, n_int.ptr, span.ptr);
+  while (true) {
+    const int last = std::min(level + batch, kMaxLevels);
+    for (; level < last; ++level) {
+      k_level_plan<<<blocks(level), kEncodeThreads, 0, s>>>(bin.nodes.ptr, sah ? dp.ptr : nullptr, sah ? width : 0, w,
+                                                            level);
+      k_level_scan<<<1, 1024, 0, s>>>(w, level, (uint32_t)std::min<size_t>(rec_cap, 0xFFFFFFFFu));
+      k_level_emit<<<blocks(level), kEncodeThreads, 0, s>>>(A, w, level, words.ptr, recs.ptr);
+    }
     VT_CUDA(cudaGetLastError());
-    k_scan2<<<1, 1024, 0, s>>>(n_int.ptr, span.ptr, level_n, totals.ptr);
-    VT_CUDA(cudaGetLastError());
-    unsigned long long tot[2];
-    VT_CUDA(cudaMemcpyAsync(tot, totals.ptr, sizeof tot, cudaMemcpyDeviceToHost, s));
+    VT_CUDA(cudaMemcpyAsync(&st, state.ptr, sizeof st, cudaMemcpyDeviceToHost, s));
     VT_CUDA(cudaStreamSynchronize(s));
-    if (level_start + level_n + tot[0] > max_wide) fail(VT_ERR_BUILD, "wide encoding: more nodes than bounded");
-    if (rec_used + tot[1] > rec_cap) {
-      // grow the record array (more leaf slots than the first estimate)
-      const size_t cap = std::max<size_t>(rec_used + tot[1] + 64, rec_cap * 3 / 2);
+    if (st.stop == ~0u) fail(VT_ERR_BUILD, "wide encoding: more nodes than bounded");
+    if (st.stop) {
+      // grow the record array (more leaf slots than the first estimate) and emit the level that waited
+      level = (int)st.stop - 1;
+      const size_t cap = std::max<size_t>((size_t)st.level[level + 1].rec + 64, rec_cap * 3 / 2);
       ScratchBuffer<float> bigger(16 * cap, s);
       VT_CUDA(cudaMemsetAsync(bigger.ptr, 0, bigger.bytes(), s));
-      VT_CUDA(cudaMemcpyAsync(bigger.ptr, recs.ptr, 16 * sizeof(float) * rec_used, cudaMemcpyDeviceToDevice, s));
+      VT_CUDA(cudaMemcpyAsync(bigger.ptr, recs.ptr, 16 * sizeof(float) * (size_t)st.level[level].rec,
+                              cudaMemcpyDeviceToDevice, s));
       recs = std::move(bigger);
       rec_cap = cap;
+      VT_CUDA(cudaMemsetAsync(&state.ptr->stop, 0, sizeof(uint32_t), s));
+      k_level_emit<<<blocks(level), kEncodeThreads, 0, s>>>(A, w, level, words.ptr, recs.ptr);
+      VT_CUDA(cudaGetLastError());
+      ++level;
     }
-    k_level_emit<<<blocks, 128, 0, s>>>(A, cur->ptr, level_n, plan.ptr, n_int.ptr, span.ptr, level_start, rec_used,
-                                        words.ptr, recs.ptr, nxt->ptr, err.ptr);
-    VT_CUDA(cudaGetLastError());
-    level_start += level_n;
-    rec_used += (uint32_t)tot[1];
-    level_n = (uint32_t)tot[0];
-    std::swap(cur, nxt);
+    if (level >= kMaxLevels || st.level[level].n == 0) break;
+    batch = 3;
   }
-  int bad = 0;
-  VT_CUDA(cudaMemcpyAsync(&bad, err.ptr, sizeof bad, cudaMemcpyDeviceToHost, s));
-  VT_CUDA(cudaStreamSynchronize(s));
+  while (depth < level && st.level[depth].n) ++depth;
+  const uint32_t level_start = st.level[depth].start, rec_used = st.level[depth].rec;
+  const uint32_t bad = st.err;
   if (bad) fail(VT_ERR_BUILD, "leaf records exceed 2^30");
   out.depth = depth;
   if (host_copy) {
