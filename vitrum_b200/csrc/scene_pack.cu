@@ -191,20 +191,160 @@ void append_mesh(const vt_mesh_desc& md, size_t m, size_t material_count, std::v
   }
 }
 
-// The engine's tree over vertices pos (4 floats each) and triangles idx (4
-// u32 each): the binned-SAH build and the SAH-optimal 8-wide encoding, on the
-// GPU or on the host (the same words either way).  With dev (GPU builds), the
-// tree stays there, its records carrying their materials' flags, and bin holds
-// the root alone.
-static void build_tree(const SceneBuild& sb, const std::vector<float>& pos, const std::vector<uint32_t>& idx,
-                       const uint32_t* tri_mat, uint32_t node_base, uint32_t rec_base, int max_leaf,
-                       BinaryBvhHost& bin, WideBvhHost& wide, WideBvhDevice* dev = nullptr,
-                       const std::vector<uint32_t>* mat_flags = nullptr) {
+// ---------------------------------------------------------------- geometry on the device
+namespace {
+
+struct MeshSpan {
+  uint32_t v0, t0, verts, material;  // first vertex and triangle in the scene's arrays, own vertices, material
+};
+// A scene's vertices (4 floats each), triangles (4 u32 each) and triangle
+// materials on the device, as append_mesh lays them out.
+struct DeviceGeometry {
+  ScratchBuffer<float> pos;
+  ScratchBuffer<uint32_t> idx, mat;
+  size_t nvert = 0, ntri = 0;
+};
+
+// One thread per vertex, then one per triangle; bad: something append_mesh refuses.
+__global__ void __launch_bounds__(256) k_pack_geometry(const float* __restrict__ raw_pos,
+                                                       const uint32_t* __restrict__ raw_idx,
+                                                       const MeshSpan* __restrict__ spans, uint32_t n_spans,
+                                                       size_t nvert, size_t ntri, float4* __restrict__ pos,
+                                                       uint4* __restrict__ idx, uint32_t* __restrict__ mat,
+                                                       uint32_t* __restrict__ bad) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < nvert) {
+    const float x = raw_pos[3 * i], y = raw_pos[3 * i + 1], z = raw_pos[3 * i + 2];
+    if (!isfinite(x) || !isfinite(y) || !isfinite(z)) atomicOr(bad, 1u);
+    pos[i] = make_float4(x, y, z, 0.0f);
+  } else if (i - nvert < ntri) {
+    const size_t t = i - nvert;
+    uint32_t lo = 0, hi = n_spans - 1;  // the last mesh that starts at or before t (empty ones start with the next)
+    while (lo < hi) {
+      const uint32_t mid = (lo + hi + 1) >> 1;
+      if (spans[mid].t0 <= t) lo = mid; else hi = mid - 1;
+    }
+    const MeshSpan m = spans[lo];
+    const uint32_t a = raw_idx[3 * t], b = raw_idx[3 * t + 1], c = raw_idx[3 * t + 2];
+    if (a >= m.verts || b >= m.verts || c >= m.verts) atomicOr(bad, 1u);
+    idx[t] = make_uint4(m.v0 + a, m.v0 + b, m.v0 + c, 0u);
+    mat[t] = m.material;
+  }
+}
+
+// Meshes of fewer triangles than this on average are appended on the host: two
+// copies a mesh cost more than its triangles (about 15 ns each there).
+constexpr size_t kDeviceMeshTriangles = 512;
+
+// The scene's geometry copied to the device and packed there: 262,146 triangles
+// in 0.5 ms, where validating and rebasing them on the host, page by fresh page,
+// and uploading the result took 5 ms.  False: left to append_mesh, which also
+// names what is wrong with a mesh.
+bool pack_geometry_gpu(const vt_scene_desc* sc, const SceneBuild& sb, DeviceGeometry& g) {
+  size_t nv = 0, nt = 0;
+  std::vector<MeshSpan> spans(sc->mesh_count);
+  for (size_t m = 0; m < sc->mesh_count; ++m) {
+    const vt_mesh_desc& md = sc->meshes[m];
+    if (md.material >= sc->material_count || (md.vertex_count && !md.positions) || (md.triangle_count && !md.indices))
+      return false;
+    if (nv + md.vertex_count >= 0xFFFFFFFFull || nt + md.triangle_count >= 0xFFFFFFFFull) return false;
+    spans[m] = {(uint32_t)nv, (uint32_t)nt, (uint32_t)md.vertex_count, (uint32_t)md.material};
+    nv += md.vertex_count;
+    nt += md.triangle_count;
+  }
+  if (nt == 0 || nt < kDeviceMeshTriangles * sc->mesh_count) return false;
+  DeviceScope ds(sb.device);
+  cudaStream_t s = sb.stream;
+  ScratchBuffer<float> raw_pos(3 * nv + 1, s);
+  ScratchBuffer<uint32_t> raw_idx(3 * nt, s), bad(1, s);
+  ScratchBuffer<MeshSpan> dspans(spans.size(), s);
+  g.pos.resize(4 * nv + 4, s);
+  g.idx.resize(4 * nt, s);
+  g.mat.resize(nt, s);
+  g.nvert = nv;
+  g.ntri = nt;
+  VT_CUDA(cudaMemsetAsync(bad.ptr, 0, sizeof(uint32_t), s));
+  VT_CUDA(cudaMemcpyAsync(dspans.ptr, spans.data(), dspans.bytes(), cudaMemcpyHostToDevice, s));
+  for (size_t m = 0; m < sc->mesh_count; ++m) {
+    const vt_mesh_desc& md = sc->meshes[m];
+    if (md.vertex_count)
+      VT_CUDA(cudaMemcpyAsync(raw_pos.ptr + 3 * (size_t)spans[m].v0, md.positions, 12 * md.vertex_count,
+                              cudaMemcpyHostToDevice, s));
+    if (md.triangle_count)
+      VT_CUDA(cudaMemcpyAsync(raw_idx.ptr + 3 * (size_t)spans[m].t0, md.indices, 12 * md.triangle_count,
+                              cudaMemcpyHostToDevice, s));
+  }
+  k_pack_geometry<<<(unsigned)((nv + nt + 255) / 256), 256, 0, s>>>(
+      raw_pos.ptr, raw_idx.ptr, dspans.ptr, (uint32_t)spans.size(), nv, nt, reinterpret_cast<float4*>(g.pos.ptr),
+      reinterpret_cast<uint4*>(g.idx.ptr), g.mat.ptr, bad.ptr);
+  VT_CUDA(cudaGetLastError());
+  uint32_t flagged = 0;
+  VT_CUDA(cudaMemcpyAsync(&flagged, bad.ptr, sizeof flagged, cudaMemcpyDeviceToHost, s));
+  VT_CUDA(cudaStreamSynchronize(s));
+  return !flagged;
+}
+
+// Geometry appended on the host, to the device.
+void upload_geometry(const SceneBuild& sb, const std::vector<float>& pos, const std::vector<uint32_t>& idx,
+                     const std::vector<uint32_t>& mat, DeviceGeometry& g) {
+  DeviceScope ds(sb.device);
+  cudaStream_t s = sb.stream;
+  g.nvert = pos.size() / 4;
+  g.ntri = mat.size();
+  g.pos.resize(pos.size() + 4, s);
+  g.idx.resize(idx.size() + 4, s);
+  g.mat.resize(mat.size() + 1, s);
+  if (!pos.empty()) VT_CUDA(cudaMemcpyAsync(g.pos.ptr, pos.data(), pos.size() * 4, cudaMemcpyHostToDevice, s));
+  if (!idx.empty()) VT_CUDA(cudaMemcpyAsync(g.idx.ptr, idx.data(), idx.size() * 4, cudaMemcpyHostToDevice, s));
+  if (!mat.empty()) VT_CUDA(cudaMemcpyAsync(g.mat.ptr, mat.data(), mat.size() * 4, cudaMemcpyHostToDevice, s));
+}
+
+// Options of the engine's trees and their SAH-optimal collapse.
+BuildOptions tree_options(int max_leaf) {
   BuildOptions bo;
   bo.max_leaf = max_leaf;
   bo.bins = kEngineBins;
+  return bo;
+}
+WideCollapse tree_collapse(const SceneBuild& sb) {
   WideCollapse collapse = kEngineCollapse;
   collapse.width = sb.bvh_width;
+  return collapse;
+}
+
+// The engine's tree over device geometry, left on the device: its records carry
+// their materials' flags, and bin holds the root alone.
+void build_tree_device(const SceneBuild& sb, const float* d_pos, size_t nvert, const uint32_t* d_idx,
+                       const uint32_t* d_mat, size_t ntri, int max_leaf, const std::vector<uint32_t>& mat_flags,
+                       BinaryBvhHost& bin, WideBvhDevice& dev) {
+  DeviceScope ds(sb.device);
+  cudaStream_t s = sb.stream;
+  const WideCollapse collapse = tree_collapse(sb);
+  BinaryBvhDevice bd;
+  bin = build_binary_gpu(d_pos, 4 * nvert, d_idx, 4 * ntri, tree_options(max_leaf), s, &bd, false);
+  ScratchBuffer<uint32_t> dflags;
+  if (!mat_flags.empty()) {
+    dflags.resize(mat_flags.size(), s);
+    VT_CUDA(cudaMemcpyAsync(dflags.ptr, mat_flags.data(), dflags.bytes(), cudaMemcpyHostToDevice, s));
+  }
+  encode_wide_gpu(bd, d_pos, 4, d_idx, 4, d_mat, 0, 0, &collapse, nullptr, s, &dev, false, dflags.ptr);
+  if (bd.n_nodes) {
+    bin.nodes.resize(1);
+    VT_CUDA(cudaMemcpyAsync(bin.nodes.data(), bd.nodes.ptr, sizeof(BinaryNode), cudaMemcpyDeviceToHost, s));
+  }
+  VT_CUDA(cudaStreamSynchronize(s));
+}
+
+}  // namespace
+
+// The engine's tree over vertices pos (4 floats each) and triangles idx (4
+// u32 each): the binned-SAH build and the SAH-optimal 8-wide encoding, on the
+// GPU or on the host (the same words either way).
+static void build_tree(const SceneBuild& sb, const std::vector<float>& pos, const std::vector<uint32_t>& idx,
+                       const uint32_t* tri_mat, uint32_t node_base, uint32_t rec_base, int max_leaf,
+                       BinaryBvhHost& bin, WideBvhHost& wide) {
+  const BuildOptions bo = tree_options(max_leaf);
+  const WideCollapse collapse = tree_collapse(sb);
   const size_t ntri = idx.size() / 4;
   if (sb.gpu) {
     DeviceScope ds(sb.device);
@@ -214,19 +354,9 @@ static void build_tree(const SceneBuild& sb, const std::vector<float>& pos, cons
     if (!idx.empty()) VT_CUDA(cudaMemcpyAsync(didx.ptr, idx.data(), idx.size() * 4, cudaMemcpyHostToDevice, sb.stream));
     if (ntri && tri_mat) VT_CUDA(cudaMemcpyAsync(dmat.ptr, tri_mat, ntri * 4, cudaMemcpyHostToDevice, sb.stream));
     BinaryBvhDevice bd;
-    bin = build_binary_gpu(dpos.ptr, pos.size(), didx.ptr, idx.size(), bo, sb.stream, &bd, dev == nullptr);
-    ScratchBuffer<uint32_t> dflags;
-    if (dev && mat_flags && !mat_flags->empty()) {
-      dflags.resize(mat_flags->size(), sb.stream);
-      VT_CUDA(cudaMemcpyAsync(dflags.ptr, mat_flags->data(), dflags.bytes(), cudaMemcpyHostToDevice, sb.stream));
-    }
+    bin = build_binary_gpu(dpos.ptr, pos.size(), didx.ptr, idx.size(), bo, sb.stream, &bd);
     wide = encode_wide_gpu(bd, dpos.ptr, 4, didx.ptr, 4, tri_mat ? dmat.ptr : nullptr, node_base, rec_base,
-                           &collapse, nullptr, sb.stream, dev, dev == nullptr, dflags.ptr);
-    if (dev && bd.n_nodes) {
-      bin.nodes.resize(1);
-      VT_CUDA(cudaMemcpyAsync(bin.nodes.data(), bd.nodes.ptr, sizeof(BinaryNode), cudaMemcpyDeviceToHost, sb.stream));
-      VT_CUDA(cudaStreamSynchronize(sb.stream));
-    }
+                           &collapse, nullptr, sb.stream);
   } else {
     bin = build_binary_host(pos.data(), pos.size(), idx.data(), idx.size(), bo);
     wide = encode_wide(bin, pos.data(), 4, idx.data(), 4, tri_mat, node_base, rec_base, &collapse);
@@ -288,7 +418,12 @@ PackedScene pack_scene(const vt_scene_desc* sc, uint32_t node_base, uint32_t rec
   PackedScene p;
   std::vector<float> pos;
   std::vector<uint32_t> idx, tri_mat;
-  for (size_t m = 0; m < sc->mesh_count; ++m) append_mesh(sc->meshes[m], m, sc->material_count, pos, idx, tri_mat);
+  DeviceGeometry geo;
+  p.on_device = sb.gpu && sb.keep && !sb.validate && !sc->instance_count;
+  if (!p.on_device || !pack_geometry_gpu(sc, sb, geo)) {
+    for (size_t m = 0; m < sc->mesh_count; ++m) append_mesh(sc->meshes[m], m, sc->material_count, pos, idx, tri_mat);
+    if (p.on_device) upload_geometry(sb, pos, idx, tri_mat, geo);
+  }
   // materials
   std::vector<pt::Material> mats(sc->material_count);
   for (size_t i = 0; i < sc->material_count; ++i) {
@@ -317,7 +452,7 @@ PackedScene pack_scene(const vt_scene_desc* sc, uint32_t node_base, uint32_t rec
     if (d.flags & ~3u) fail(VT_ERR_INVALID_ARGUMENT, "material " + std::to_string(i) + " has unknown flags");
     m.flags = d.flags;
   }
-  const size_t ntri = tri_mat.size();
+  const size_t ntri = p.on_device ? geo.ntri : tri_mat.size();
   // geometry
   const bool two_level = sc->instance_count > 0;
   if (two_level && !sc->instances) fail(VT_ERR_INVALID_ARGUMENT, "instances is null");
@@ -327,11 +462,14 @@ PackedScene pack_scene(const vt_scene_desc* sc, uint32_t node_base, uint32_t rec
   uint32_t root = 0;
   if (!two_level) {
     WideBvhHost w;
-    p.on_device = sb.gpu && sb.keep && !sb.validate;
-    std::vector<uint32_t> flags(mats.size());
-    for (size_t i = 0; i < mats.size(); ++i) flags[i] = mats[i].flags;
-    build_tree(sb, pos, idx, tri_mat.data(), node_base, rec_base, max_leaf, p.binary, w, p.on_device ? &p.dev : nullptr,
-               &flags);
+    if (p.on_device) {
+      std::vector<uint32_t> flags(mats.size());
+      for (size_t i = 0; i < mats.size(); ++i) flags[i] = mats[i].flags;
+      build_tree_device(sb, geo.pos.ptr, geo.nvert, geo.idx.ptr, geo.mat.ptr, ntri, max_leaf, flags, p.binary, p.dev);
+      w.depth = p.dev.depth;
+    } else {
+      build_tree(sb, pos, idx, tri_mat.data(), node_base, rec_base, max_leaf, p.binary, w);
+    }
     node_words = std::move(w.nodes);
     rec_floats = std::move(w.tris);
     depth = w.depth;
@@ -401,25 +539,28 @@ PackedScene pack_scene(const vt_scene_desc* sc, uint32_t node_base, uint32_t rec
   std::vector<float4> em;
   std::vector<float> cdf;
   double total = 0.0;
-  for (size_t t = 0; t < ntri && !two_level; ++t) {
-    if (!mats[tri_mat[t]].emissive) continue;
-    const float* a = &pos[4 * idx[4 * t]];
-    const float* b = &pos[4 * idx[4 * t + 1]];
-    const float* c = &pos[4 * idx[4 * t + 2]];
-    const double e1[3] = {(double)b[0] - a[0], (double)b[1] - a[1], (double)b[2] - a[2]};
-    const double e2[3] = {(double)c[0] - a[0], (double)c[1] - a[1], (double)c[2] - a[2]};
-    const double cx = e1[1] * e2[2] - e1[2] * e2[1], cy = e1[2] * e2[0] - e1[0] * e2[2],
-                 cz = e1[0] * e2[1] - e1[1] * e2[0];
-    const double area = 0.5 * std::sqrt(cx * cx + cy * cy + cz * cz);
-    if (!(area > 0.0)) continue;
-    uint32_t mb = tri_mat[t];
-    float mf;
-    std::memcpy(&mf, &mb, 4);
-    em.push_back(make_float4(a[0], a[1], a[2], mf));
-    em.push_back(make_float4(b[0], b[1], b[2], (float)area));
-    em.push_back(make_float4(c[0], c[1], c[2], 0.0f));
-    total += area;
-    cdf.push_back((float)total);
+  for (size_t m = 0; m < sc->mesh_count && !two_level; ++m) {
+    const vt_mesh_desc& md = sc->meshes[m];
+    if (!mats[md.material].emissive) continue;
+    for (size_t t = 0; t < md.triangle_count; ++t) {
+      const float* a = md.positions + 3 * (size_t)md.indices[3 * t];
+      const float* b = md.positions + 3 * (size_t)md.indices[3 * t + 1];
+      const float* c = md.positions + 3 * (size_t)md.indices[3 * t + 2];
+      const double e1[3] = {(double)b[0] - a[0], (double)b[1] - a[1], (double)b[2] - a[2]};
+      const double e2[3] = {(double)c[0] - a[0], (double)c[1] - a[1], (double)c[2] - a[2]};
+      const double cx = e1[1] * e2[2] - e1[2] * e2[1], cy = e1[2] * e2[0] - e1[0] * e2[2],
+                   cz = e1[0] * e2[1] - e1[1] * e2[0];
+      const double area = 0.5 * std::sqrt(cx * cx + cy * cy + cz * cz);
+      if (!(area > 0.0)) continue;
+      const uint32_t mb = md.material;
+      float mf;
+      std::memcpy(&mf, &mb, 4);
+      em.push_back(make_float4(a[0], a[1], a[2], mf));
+      em.push_back(make_float4(b[0], b[1], b[2], (float)area));
+      em.push_back(make_float4(c[0], c[1], c[2], 0.0f));
+      total += area;
+      cdf.push_back((float)total);
+    }
   }
   for (float& x : cdf) x = (float)(x / total);
   if (!cdf.empty()) cdf.back() = 1.0f;
