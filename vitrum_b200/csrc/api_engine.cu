@@ -63,6 +63,7 @@ struct vt_engine {
   bool has_scene = false;
   vt::BinaryBvhHost binary;
   vt::PoolBuffer<uint4> nodes;
+  size_t nodes_u4 = 0;             // words in use (an instance update may leave room behind them)
   vt::PoolBuffer<float4> tris;
   int wide_depth = 1;
   int stack_depth = 16;            // traversal stack entries the scene needs
@@ -238,6 +239,7 @@ void set_scene(vt_engine* e, const vt_scene_desc* sc) {
   // commit
   e->drop_graphs();
   e->nodes = std::move(n.nodes);
+  e->nodes_u4 = n_u4;
   e->tris = std::move(n.tris);
   e->insts = std::move(n.insts);
   e->inst_table = std::move(n.inst_table);
@@ -337,32 +339,53 @@ void update_instances(vt_engine* e, const vt_instance_desc* insts, size_t n, boo
   vt::WideBvhHost tw = vt::encode_top_level(sb, tl, placed.recs, e->tlas_root);
   cudaStream_t s = e->stream;
   VT_CUDA(cudaStreamSynchronize(s));
-  e->drop_graphs();
+  // The captured graphs hold these pointers, the stack bound and, where nodes are
+  // staged or queues traced in spatial order, the node count and the scene's
+  // bounds.  They stay while those do: arrays grow with room behind them and the
+  // bound never shrinks, because a refitted top level's encoding varies a little
+  // in size from frame to frame (0.7 ms of a moving frame was their re-capture).
+  struct DropUnlessKept {
+    vt_engine* e;
+    const void* nodes;
+    const void* insts;
+    const void* table;
+    size_t nodes_u4;
+    int stack;
+    bool done = false;
+    ~DropUnlessKept() {
+      if (!done || nodes != e->nodes.ptr || insts != e->insts.ptr || table != e->inst_table.ptr ||
+          stack != e->stack_depth || e->sort_rays >= 2 || (e->trace_stage_nodes && nodes_u4 != e->nodes_u4))
+        e->drop_graphs();
+    }
+  } held{e, e->nodes.ptr, e->insts.ptr, e->inst_table.ptr, e->nodes_u4, e->stack_depth};
   const size_t blas_u4 = (size_t)e->tlas_root * 5, tlas_u4 = tw.nodes.size() / 4;
-  if (blas_u4 + tlas_u4 != e->nodes.count) {
+  if (blas_u4 + tlas_u4 > e->nodes.count) {
     vt::PoolBuffer<uint4> grown;
-    grown.resize(blas_u4 + tlas_u4, s);
+    grown.resize(blas_u4 + tlas_u4 + tlas_u4 / 4, s);
     if (blas_u4)
       VT_CUDA(cudaMemcpyAsync(grown.ptr, e->nodes.ptr, blas_u4 * sizeof(uint4), cudaMemcpyDeviceToDevice, s));
     VT_CUDA(cudaStreamSynchronize(s));
     e->nodes = std::move(grown);
   }
+  e->nodes_u4 = blas_u4 + tlas_u4;
   VT_CUDA(cudaMemcpyAsync(e->nodes.ptr + blas_u4, tw.nodes.data(), tw.nodes.size() * 4, cudaMemcpyHostToDevice, s));
   std::vector<float4> il(tw.tris.size() / 4), it(n * 4), ir(placed.rows.size() / 4);
   if (!il.empty()) std::memcpy(il.data(), tw.tris.data(), tw.tris.size() * 4);
   std::memcpy(it.data(), placed.recs.data(), n * sizeof(vt::InstanceRecord));
   if (!ir.empty()) std::memcpy(ir.data(), placed.rows.data(), placed.rows.size() * 4);
-  upload(e->insts, il, s);
+  if (il.size() > e->insts.count) e->insts.resize(il.size() + il.size() / 4);
+  if (!il.empty()) VT_CUDA(cudaMemcpyAsync(e->insts.ptr, il.data(), il.size() * sizeof(float4), cudaMemcpyHostToDevice, s));
   upload(e->inst_table, it, s);
   upload(e->inst_l2w, ir, s);
   VT_CUDA(cudaStreamSynchronize(s));
   e->binary = std::move(tl);
   e->wide_depth = tw.depth + e->blas_depth;
-  e->stack_depth = 2 * e->wide_depth + 6;
+  e->stack_depth = std::max(e->stack_depth, 2 * e->wide_depth + 6);
   e->view.nodes = e->nodes.ptr;
   e->view.stack_depth = e->stack_depth;
   e->view.insts = e->insts.ptr;
   e->view.inst_table = e->inst_table.ptr;
+  held.done = true;
   reset_accumulation(e);
   VT_CUDA(cudaStreamSynchronize(e->stream));
 }
@@ -413,13 +436,14 @@ void update_mesh(vt_engine* e, size_t m, const vt_mesh_desc* md, bool rebuild) {
   e->blas_depth = *std::max_element(e->blas_depths.begin(), e->blas_depths.end());
   e->ntri += (int64_t)md->triangle_count - (int64_t)e->mesh_tris[m];
   e->mesh_tris[m] = md->triangle_count;
-  const size_t tlas_u4 = e->nodes.count - (size_t)old_tlas_root * 5;
+  const size_t tlas_u4 = e->nodes_u4 - (size_t)old_tlas_root * 5;
   // upload the bottom levels and records; the top level follows in update_instances
   cudaStream_t s = e->stream;
   VT_CUDA(cudaStreamSynchronize(s));
   e->drop_graphs();
   const size_t blas_u4 = e->blas_words.size() / 4;
-  e->nodes.resize(blas_u4 + tlas_u4, s);  // the top level's part is written by update_instances
+  e->nodes_u4 = blas_u4 + tlas_u4;
+  e->nodes.resize(e->nodes_u4, s);  // the top level's part is written by update_instances
   VT_CUDA(cudaMemcpyAsync(e->nodes.ptr, e->blas_words.data(), e->blas_words.size() * 4, cudaMemcpyHostToDevice, s));
   e->tris.resize(std::max<size_t>(e->rec_host.size() / 4, 1), s);
   VT_CUDA(cudaMemcpyAsync(e->tris.ptr, e->rec_host.data(), e->rec_host.size() * 4, cudaMemcpyHostToDevice, s));
@@ -691,7 +715,7 @@ void record_wave(vt_engine* e, uint32_t spp_wave, uint32_t bounces, cudaStream_t
     t.status = e->trace_status.ptr;
     t.counter = e->trace_counter.ptr;
     t.stack_depth = e->stack_depth;
-    t.node_count = e->nodes.count / 5;
+    t.node_count = e->nodes_u4 / 5;
     t.stage_nodes = e->trace_stage_nodes;
     t.stage_wait_cycles = e->debug_wait_cycles;
     t.insts = e->view.insts;
@@ -1242,7 +1266,7 @@ vt_status vt_pick(vt_engine* e, float x, float y, int32_t* out_triangle) {
     t.status = e->pick_status.ptr;
     t.counter = e->pick_counter.ptr;
     t.stack_depth = e->stack_depth;
-    t.node_count = e->nodes.count / 5;
+    t.node_count = e->nodes_u4 / 5;
     t.stage_nodes = e->trace_stage_nodes;
     t.stage_wait_cycles = e->debug_wait_cycles;
     t.insts = e->view.insts;
@@ -1273,7 +1297,7 @@ vt_status vt_engine_export_scene(const vt_engine* e, uint32_t* node_words, size_
     if (!e) fail(VT_ERR_INVALID_ARGUMENT, "engine is null");
     if (!e->has_scene) fail(VT_ERR_STATE, "export before setScene");
     vt::DeviceScope ds(e->device);
-    const size_t nw = e->nodes.count * 4, nf = e->tris.count * 4;
+    const size_t nw = e->nodes_u4 * 4, nf = e->tris.count * 4;
     if (out_words) *out_words = nw;
     if (out_floats) *out_floats = nf;
     VT_CUDA(cudaStreamSynchronize(e->stream));
@@ -1330,7 +1354,7 @@ vt_status vt_trace_rays(vt_engine* e, const vt_ray* rays, size_t n, vt_hit* hits
     t.status = e->q_status.ptr;
     t.counter = e->q_counter.ptr;
     t.stack_depth = e->stack_depth;
-    t.node_count = e->nodes.count / 5;
+    t.node_count = e->nodes_u4 / 5;
     t.stage_nodes = e->trace_stage_nodes;
     t.stage_wait_cycles = e->debug_wait_cycles;
     t.insts = e->view.insts;

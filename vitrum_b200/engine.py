@@ -299,6 +299,21 @@ class Camera:
         return view.T.reshape(-1).astype(np.float32), proj.T.reshape(-1).astype(np.float32)
 
 
+_INSTANCE_DTYPE = np.dtype([("mesh", np.uint32), ("material", np.uint32), ("local_to_world", np.float32, 16)])
+
+
+def _marshal_instances(instances: Sequence["Instance"]):
+    """vt_instance_desc array (column-major matrices), at least one element."""
+    arr = (_InstanceDesc * max(1, len(instances)))()
+    if instances:
+        a = np.frombuffer(arr, _INSTANCE_DTYPE)
+        a["mesh"] = [int(i.mesh) & 0xFFFFFFFF for i in instances]
+        a["material"] = [int(i.material) & 0xFFFFFFFF for i in instances]
+        m = np.stack([np.asarray(i.local_to_world, np.float32).reshape(4, 4) for i in instances])
+        a["local_to_world"] = m.transpose(0, 2, 1).reshape(-1, 16)
+    return arr
+
+
 def _marshal_scene(scene: "Scene"):
     """(vt_scene_desc, list of arrays that must outlive the call)."""
     keep = []
@@ -320,10 +335,7 @@ def _marshal_scene(scene: "Scene"):
         env = np.ascontiguousarray(scene.environment.rgb, np.float32)
         keep.append(env)
         env_ptr, eh, ew, ei = env.ctypes.data, env.shape[0], env.shape[1], scene.environment.intensity
-    insts = (_InstanceDesc * max(1, len(scene.instances)))()
-    for i, inst in enumerate(scene.instances):
-        M = np.asarray(inst.local_to_world, np.float32).reshape(4, 4)
-        insts[i] = _InstanceDesc(int(inst.mesh), int(inst.material), (ctypes.c_float * 16)(*M.T.reshape(-1)))
+    insts = _marshal_instances(scene.instances)
     dls = (_DirectionalDesc * max(1, len(scene.directional_lights)))()
     for i, l in enumerate(scene.directional_lights):
         dls[i] = _DirectionalDesc((ctypes.c_float * 3)(*l.direction), (ctypes.c_float * 3)(*l.irradiance),
@@ -444,10 +456,7 @@ class Engine:
         instances, same count (vt_update_instances): the top level is refitted
         (refitTlasTransforms) or, with rebuild, rebuilt over the new bounds
         (rebuildTlasReuseBlas); bottom levels are kept.  Clears the accumulation."""
-        arr = (_InstanceDesc * max(1, len(instances)))()
-        for i, inst in enumerate(instances):
-            M = np.asarray(inst.local_to_world, np.float32).reshape(4, 4)
-            arr[i] = _InstanceDesc(int(inst.mesh), int(inst.material), (ctypes.c_float * 16)(*M.T.reshape(-1)))
+        arr = _marshal_instances(instances)
         N.call("vt_update_instances", self.handle, ctypes.cast(arr, ctypes.c_void_p), len(instances),
                1 if rebuild else 0)
         if self._scene is not None:
