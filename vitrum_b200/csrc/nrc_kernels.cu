@@ -99,32 +99,63 @@ __device__ __forceinline__ Cell grid_cell(const View& v, int l, float3 n01) {
   return {(uint32_t)(int)x0, (uint32_t)(int)y0, (uint32_t)(int)z0, px - x0, py - y0, pz - z0};
 }
 
-// The two features of level l at a point: trilinear blend of the 8 corner rows.
-__device__ __forceinline__ uint32_t encode_level(const View& v, int l, float3 n01) {
+// A lane pair's two points.  The pair gathers (and scatters) for both together,
+// the even lane the corners at x, the odd lane those at x + 1: the hash's x prime
+// is 1, so the two rows differ in a few low bits, and 31 of 32 pairs fall into one
+// 128-byte line (7 of 8 into one 32-byte sector), which a warp's one access then
+// touches once instead of twice.  1,048,576 queries of the 16 x 2^19 grid, bound by
+// the L1's lookups: 383 -> 326 us.
+struct PointPair {
+  float3 even, odd;  // the even and the odd lane's point
+  bool is_odd;       // this lane's place
+};
+__device__ __forceinline__ PointPair pair_points(float3 n01) {
+  const float3 o = make_float3(__shfl_xor_sync(0xFFFFFFFFu, n01.x, 1), __shfl_xor_sync(0xFFFFFFFFu, n01.y, 1),
+                               __shfl_xor_sync(0xFFFFFFFFu, n01.z, 1));
+  const bool odd = threadIdx.x & 1u;
+  return {odd ? o : n01, odd ? n01 : o, odd};
+}
+
+// The two features of level l at this lane's point: trilinear blend of the 8
+// corner rows.  Called by whole warps.
+__device__ __forceinline__ uint32_t encode_level(const View& v, int l, const PointPair& q) {
   float f0 = 0.0f, f1 = 0.0f;
   if (l < v.levels) {
-    const Cell c = grid_cell(v, l, n01);
-    const __half2* tab = v.table16 + (size_t)l * (v.table_mask + 1u);
+    const Cell ce = grid_cell(v, l, q.even), co = grid_cell(v, l, q.odd);
+    const float fx = q.is_odd ? co.fx : ce.fx, fy = q.is_odd ? co.fy : ce.fy, fz = q.is_odd ? co.fz : ce.fz;
+    const uint32_t* tab = reinterpret_cast<const uint32_t*>(v.table16 + (size_t)l * (v.table_mask + 1u));
+    const uint32_t h = q.is_odd ? 1u : 0u;
+    uint32_t e0[4], e1[4];  // rows at x and x + 1 of this lane's point
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const uint32_t cx = k & 1, cy = (k >> 1) & 1, cz = (k >> 2) & 1;
-      const float w = (cx ? c.fx : 1.0f - c.fx) * (cy ? c.fy : 1.0f - c.fy) * (cz ? c.fz : 1.0f - c.fz);
-      const uint32_t row = grid_hash(c.x + cx, c.y + cy, c.z + cz) & v.table_mask;
-      const float2 e = __half22float2(__ldg(tab + row));
-      f0 = fmaf(w, e.x, f0);
-      f1 = fmaf(w, e.y, f1);
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t cy = k & 1, cz = k >> 1;
+      const uint32_t e = __ldg(tab + (grid_hash(ce.x + h, ce.y + cy, ce.z + cz) & v.table_mask));
+      const uint32_t o = __ldg(tab + (grid_hash(co.x + h, co.y + cy, co.z + cz) & v.table_mask));
+      const uint32_t theirs = __shfl_xor_sync(0xFFFFFFFFu, q.is_odd ? e : o, 1);
+      e0[k] = q.is_odd ? theirs : e;
+      e1[k] = q.is_odd ? o : theirs;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t cy = k & 1, cz = k >> 1;
+      const float w0 = (1.0f - fx) * (cy ? fy : 1.0f - fy) * (cz ? fz : 1.0f - fz);
+      const float w1 = fx * (cy ? fy : 1.0f - fy) * (cz ? fz : 1.0f - fz);
+      const float2 a = unpack_h2(e0[k]), b = unpack_h2(e1[k]);
+      f0 = fmaf(w0, a.x, f0);
+      f1 = fmaf(w0, a.y, f1);
+      f0 = fmaf(w1, b.x, f0);
+      f1 = fmaf(w1, b.y, f1);
     }
   }
   return pack_h2(f0, f1);
 }
 
 // Encodes one record (4 float4) into 64 fp16 inputs packed as 32 half2 words.
-__device__ __forceinline__ void encode(const View& v, float4 a, float4 b, float4 c, float4 d, uint32_t (&p)[32],
-                                       float3& n01) {
-  n01 = normalise(v, a.x, a.y, a.z);
+__device__ __forceinline__ void encode(const View& v, float4 a, float4 b, float4 c, float4 d, uint32_t (&p)[32]) {
+  const PointPair q = pair_points(normalise(v, a.x, a.y, a.z));
   // all levels unrolled: the 8 x levels table gathers are independent and in flight together
 #pragma unroll
-  for (int l = 0; l < kMaxLevels; ++l) p[l] = encode_level(v, l, n01);
+  for (int l = 0; l < kMaxLevels; ++l) p[l] = encode_level(v, l, q);
   float s[16];
   sh4(a.w, b.x, b.y, s);
 #pragma unroll
@@ -140,28 +171,27 @@ __device__ __forceinline__ void encode(const View& v, float4 a, float4 b, float4
   p[31] = 0u;
 }
 
-// Scatter of the input gradient of level l's two features (already scaled)
-// into the f32 table gradient with the trilinear weights.
-__device__ __forceinline__ void scatter_level(const View& v, int l, float3 n01, float g0, float g1) {
-  if (l >= v.levels || (g0 == 0.0f && g1 == 0.0f)) return;
-  const Cell c = grid_cell(v, l, n01);
+// Scatter of the input gradient (g0, g1) of level l's two features (already
+// scaled) into the f32 table gradient with the trilinear weights, the pair for
+// its two points in turn as in the gather: the L2 takes the neighbouring rows of
+// one access as one operation per sector.  Called by whole warps; zero gradients
+// add nothing.
+__device__ __forceinline__ void scatter_level(const View& v, int l, const PointPair& q, float g0, float g1) {
+  const float p0 = __shfl_xor_sync(0xFFFFFFFFu, g0, 1), p1 = __shfl_xor_sync(0xFFFFFFFFu, g1, 1);
+  if (l >= v.levels) return;
+  const uint32_t h = q.is_odd ? 1u : 0u;
   float2* gt = v.grad_table + (size_t)l * (v.table_mask + 1u);
-  // corners x and x + 1 are neighbouring rows when x is even (the hash's x prime is
-  // 1): one 16-byte atomic then adds both, six instead of eight a level on average
-  const bool odd = c.x & 1u;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const uint32_t cy = k & 1, cz = k >> 1;
-    const float wy = cy ? c.fy : 1.0f - c.fy, wz = cz ? c.fz : 1.0f - c.fz;
-    const float w0 = (1.0f - c.fx) * wy * wz, w1 = c.fx * wy * wz;
-    const uint32_t r0 = grid_hash(c.x, c.y + cy, c.z + cz) & v.table_mask;
-    const float2 a0 = make_float2(w0 * g0, w0 * g1), a1 = make_float2(w1 * g0, w1 * g1);
-    if (odd) {
-      atomicAdd(gt + r0, a0);
-      atomicAdd(gt + (grid_hash(c.x + 1u, c.y + cy, c.z + cz) & v.table_mask), a1);
-    } else {
-      const float2 lo = (r0 & 1u) ? a1 : a0, hi = (r0 & 1u) ? a0 : a1;
-      atomicAdd(reinterpret_cast<float4*>(gt + (r0 & ~1u)), make_float4(lo.x, lo.y, hi.x, hi.y));
+  for (int s = 0; s < 2; ++s) {
+    const float a0 = (s == 1) == q.is_odd ? g0 : p0, a1 = (s == 1) == q.is_odd ? g1 : p1;
+    if (a0 == 0.0f && a1 == 0.0f) continue;
+    const Cell c = grid_cell(v, l, s ? q.odd : q.even);
+    const float wx = h ? c.fx : 1.0f - c.fx;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t cy = k & 1, cz = k >> 1;
+      const float w = wx * (cy ? c.fy : 1.0f - c.fy) * (cz ? c.fz : 1.0f - c.fz);
+      atomicAdd(gt + (grid_hash(c.x + h, c.y + cy, c.z + cz) & v.table_mask), make_float2(w * a0, w * a1));
     }
   }
 }
@@ -277,9 +307,8 @@ __global__ void __launch_bounds__(128 * T, T == 1 ? 3 : (T == 2 ? 2 : 1))
     const uint32_t i = tile * kTile + tid;
     const bool valid = i < n;
     uint32_t p[32];
-    float3 n01;
     const float4* r = recs + (size_t)(valid ? i : 0) * stride;
-    encode(v, __ldg(r), __ldg(r + 1), __ldg(r + 2), __ldg(r + 3), p, n01);
+    encode(v, __ldg(r), __ldg(r + 1), __ldg(r + 2), __ldg(r + 3), p);
     store_row(act, tid, p);
     tc::fence_async_smem();
     tc::fence_before_sync();
@@ -367,10 +396,11 @@ __device__ __forceinline__ uint4* chunk_at(uint8_t* tile, uint32_t r, uint32_t j
 // chain of twelve dependent products and epilogues, the gradient atomics -- so
 // what the four-fold warps buy is overlap.
 // Measured per 65,536-sample step (2^15 / 2^19 tables, optimiser included): one
-// warpgroup 165 / 274 us; four 160 / 265; with 16-byte atomics for the weight
-// gradients (3.6 M single ones before) and for neighbouring table rows 123 / 231;
-// one barrier a layer 120 / 228.  Of a step's 120 us the table atomics take 34
-// (6.3 M at the L2's rate), the encoding 22, the chain of products 46.
+// warpgroup 165 / 274 us; four 160 / 265; 16-byte atomics for the weight
+// gradients (3.6 M single ones before) and for table rows that share 16 bytes
+// 123 / 231; one barrier a layer 120 / 228; lane pairs for gathers and scatters
+// instead of the 16-byte table atomics 106 / 211.  The chain of products alone
+// is 46 us of that, the table atomics were 34 and the gathers 22 before the pairs.
 constexpr int kTrainGroups = 4;
 __global__ void __launch_bounds__(128 * kTrainGroups, 1)
     k_nrc_train(View v, const float4* __restrict__ samples, uint32_t n) {
@@ -409,11 +439,11 @@ __global__ void __launch_bounds__(128 * kTrainGroups, 1)
     const bool valid = i < n;
     const float4* r = samples + (size_t)(valid ? i : 0) * 5;
     const float4 ra = __ldg(r);
-    const float3 n01 = normalise(v, ra.x, ra.y, ra.z);
+    const PointPair point = pair_points(normalise(v, ra.x, ra.y, ra.z));
     {
       uint32_t p[4];
 #pragma unroll
-      for (int l = 0; l < 4; ++l) p[l] = encode_level(v, 4 * (int)part + l, n01);
+      for (int l = 0; l < 4; ++l) p[l] = encode_level(v, 4 * (int)part + l, point);
       *chunk_at(X, row, part) = make_uint4(p[0], p[1], p[2], p[3]);
       // columns 32 + 8 part: the spherical harmonics' halves, then the surface features
       if (part < 2) {
@@ -551,12 +581,12 @@ __global__ void __launch_bounds__(128 * kTrainGroups, 1)
       }
       if (__syncthreads_or(!ok)) { failed = true; break; }
       phase ^= 1u;
-      if (l == 0 && valid) {
+      if (l == 0) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const float g0 = __uint_as_float((part & 1u) ? acc[8 + 2 * q] : acc[2 * q]) * inv_n;
           const float g1 = __uint_as_float((part & 1u) ? acc[9 + 2 * q] : acc[2 * q + 1]) * inv_n;
-          scatter_level(v, 4 * (int)part + q, n01, g0, g1);
+          scatter_level(v, 4 * (int)part + q, point, valid ? g0 : 0.0f, valid ? g1 : 0.0f);
         }
       }
     }
@@ -693,13 +723,13 @@ void launch_infer(const View& v, const float4* records, uint32_t rec_stride_f4, 
                   float* rgb_out, float4* radiance, int tiles_per_cta, cudaStream_t s) {
   if (n == 0) return;
   // a batch of fewer tiles than SMs x T gets fewer tiles per CTA instead of idle SMs
-  // (1,000 to 18,944 queries: 31 -> 18 us; 40,000: 33 -> 27 us)
+  // (1,000 to 18,944 queries: 31 -> 17 us; 40,000: 33 -> 24 us)
   const uint32_t tiles = (n + kTile - 1) / kTile, sms = (uint32_t)sm_count();
   tiles_per_cta = (int)std::min<uint32_t>((uint32_t)tiles_per_cta, (tiles + sms - 1) / sms);
   // tiles in flight per CTA: 1 to 4 (65 to 113 KB of shared memory).  Under the default
   // carve-out one CTA runs per SM, which keeps most of the unified L1 for the hash-table gathers:
   // asking for the largest shared-memory carve-out (three or two CTAs per SM) made two tiles per
-  // CTA slower (0.47 -> 0.82 ms for 1,048,576 queries)
+  // CTA slower (0.47 -> 0.82 ms for 1,048,576 queries), and so do five or six (0.335 against 0.326)
   if (tiles_per_cta >= 4) launch_infer_t<4>(v, records, rec_stride_f4, n_dev, n, rgb_out, radiance, s);
   else if (tiles_per_cta == 3) launch_infer_t<3>(v, records, rec_stride_f4, n_dev, n, rgb_out, radiance, s);
   else if (tiles_per_cta == 2) launch_infer_t<2>(v, records, rec_stride_f4, n_dev, n, rgb_out, radiance, s);
