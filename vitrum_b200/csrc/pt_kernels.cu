@@ -536,8 +536,6 @@ __device__ __forceinline__ void nrc_features(const Material& m, float3 P, float3
 }
 
 // ---------------------------------------------------------------- shade
-// 8 resident blocks per SM (64 registers, some spilled to L1): the kernel is
-// load-latency bound, and occupancy beats spill-free code here.
 // ---------------------------------------------------------------- auxiliary outputs
 // projectToNdc (kernelCore.wgsl.ts:28-42): clip = M (p, 1) scaled by its
 // largest magnitude, (2, 2) when that is zero or not finite or w <= 0.
@@ -592,12 +590,23 @@ __global__ void k_aux_first_hit(SceneView sc, FrameView f, WaveBuffers w) {
   a.motion[pix] = make_float4((c.x - q.x) * 0.5f * (float)f.width, (c.y - q.y) * 0.5f * (float)f.height, 0.0f, 1.0f);
 }
 
-__global__ void __launch_bounds__(128, 8) k_shade(SceneView sc0, FrameView f, WaveBuffers w, int cur, uint32_t bounce) {
+// 32 warps per SM (64 registers, some spilled to L1): the kernel is load-latency
+// bound, and occupancy beats spill-free code here.  Its second bound is
+// instruction supply (a warp runs kilobytes of straight-line code once per path):
+// the warps of a CTA start each path together, so that they read the same code.
+// Measured per frame (box room unsorted / sorted by material / instanced cloud):
+// CTAs of 4 warps on their own 6.9 / 5.7 / 3.1 ms, together 6.4 / 5.7 / 3.0; of 8
+// 6.3 / 5.6 / 2.9; of 16, two per SM, 6.2 / 5.3 / 3.0; of 32 6.5 / 5.7 / 3.2; a
+// second meeting before the queues are written 6.3 / 5.5 / 3.0.
+constexpr unsigned kShadeThreads = 512;
+__global__ void __launch_bounds__(kShadeThreads, 2)
+    k_shade(SceneView sc0, FrameView f, WaveBuffers w, int cur, uint32_t bounce) {
   const int nxt = cur ^ 1;
   const uint32_t n = w.counters[cur];
   const uint32_t lane = threadIdx.x & 31u;
-  for (uint32_t base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; base < n;
-       base += gridDim.x * blockDim.x) {
+  for (uint32_t first = blockIdx.x * blockDim.x; first < n; first += gridDim.x * blockDim.x) {
+    __syncthreads();
+    const uint32_t base = first + (threadIdx.x & ~31u);
     const uint32_t i = base + lane;
     const bool valid = i < n;
     bool alive = false, shadow = false, query = false;
@@ -1118,8 +1127,10 @@ void launch_shade(const SceneView& sc, const FrameView& f, const WaveBuffers& w,
                   uint32_t capacity, cudaStream_t s) {
   cudaMemsetAsync(w.counters + (cur ^ 1), 0, sizeof(uint32_t), s);
   cudaMemsetAsync(w.counters + kCntShadow, 0, sizeof(uint32_t), s);
-  const unsigned g = grid_for(capacity, 128) < 148 * 16 ? grid_for(capacity, 128) : 148 * 16;
-  k_shade<<<g, 128, 0, s>>>(sc, f, w, cur, bounce);
+  // a wave that does not fill the SMs with large CTAs goes out in small ones
+  const unsigned block = capacity >= 2u * 148u * kShadeThreads ? kShadeThreads : 128u, most = 148u * 2048u / block;
+  const unsigned g = grid_for(capacity, block) < most ? grid_for(capacity, block) : most;
+  k_shade<<<g, block, 0, s>>>(sc, f, w, cur, bounce);
 }
 
 void launch_shadow_resolve(const WaveBuffers& w, uint32_t capacity, cudaStream_t s) {
