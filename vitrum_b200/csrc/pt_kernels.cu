@@ -535,7 +535,6 @@ __device__ __forceinline__ void nrc_features(const Material& m, float3 P, float3
   q[3] = make_float4(dif.z, spe.x, spe.y, spe.z);
 }
 
-// ---------------------------------------------------------------- shade
 // ---------------------------------------------------------------- auxiliary outputs
 // projectToNdc (kernelCore.wgsl.ts:28-42): clip = M (p, 1) scaled by its
 // largest magnitude, (2, 2) when that is zero or not finite or w <= 0.
