@@ -8,8 +8,9 @@ import dataclasses
 import numpy as np
 import pytest
 
+from vitrum_b200 import _native as N
 from vitrum_b200 import scenes
-from vitrum_b200.engine import Engine, Instance
+from vitrum_b200.engine import Engine, Instance, debug_fail_device_allocation
 
 pytestmark = pytest.mark.gpu
 
@@ -54,3 +55,35 @@ def test_frames_after_updates(cuda, tuning):
         assert all(np.array_equal(x, y) for x, y in zip(a.export_scene(), b.export_scene())), k
         b.dispose()
     a.dispose()
+
+
+def test_failed_update_keeps_the_scene(cuda):
+    """An update that runs out of device memory, at any of its allocations (the
+    first scattering outgrows the arrays), leaves the frame as it was."""
+    sc, cam = scenes.instanced_cloud(n_instances=37, seed=5, sphere_levels=(1, 2, 2, 3), torus_segments=(16, 8),
+                                     cube_cells=(2, 3, 4))
+
+    def frame(e):
+        e.reset()
+        e.render_frame(cam, 48, 32, samples=4, frame_seed=9)
+        return e.capture_frame()
+
+    e = Engine(max_bounces=3, wave_paths=1 << 16, debug=True)
+    e.set_scene(sc)
+    want = frame(e)
+    stages = 0
+    for k in range(1, 200):
+        debug_fail_device_allocation(k)
+        try:
+            e.update_instances(_placements(sc.instances, 2), True)
+        except N.VtError as err:
+            assert err.status == 4 and "injected" in str(err)
+            stages += 1
+            assert np.array_equal(frame(e), want), k
+            continue
+        finally:
+            debug_fail_device_allocation(0)
+        break
+    assert stages >= 5, stages
+    assert not np.array_equal(frame(e), want)
+    e.dispose()

@@ -327,7 +327,6 @@ void update_instances(vt_engine* e, const vt_instance_desc* insts, size_t n, boo
                                       std::to_string(n) + " (set a new scene to change the membership)");
   if (!insts) fail(VT_ERR_INVALID_ARGUMENT, "instances is null");
   vt::InstanceSet placed = vt::place_instances(insts, n, e->mats_host, e->blas_root, e->local_box);
-  if (insts != e->inst_descs.data()) e->inst_descs.assign(insts, insts + n);
   vt::BinaryBvhHost tl;
   const vt::SceneBuild sb = scene_build_of(e);
   if (rebuild) {
@@ -359,21 +358,24 @@ void update_instances(vt_engine* e, const vt_instance_desc* insts, size_t n, boo
     }
   } held{e, e->nodes.ptr, e->insts.ptr, e->inst_table.ptr, e->nodes_u4, e->stack_depth};
   const size_t blas_u4 = (size_t)e->tlas_root * 5, tlas_u4 = tw.nodes.size() / 4;
-  if (blas_u4 + tlas_u4 > e->nodes.count) {
-    vt::PoolBuffer<uint4> grown;
-    grown.resize(blas_u4 + tlas_u4 + tlas_u4 / 4, s);
+  // both arrays before either is replaced: an update that runs out of memory leaves the scene as it was
+  vt::PoolBuffer<uint4> grown;
+  DeviceBuffer<float4> more;
+  if (blas_u4 + tlas_u4 > e->nodes.count) grown.resize(blas_u4 + tlas_u4 + tlas_u4 / 4, s);
+  if (tw.tris.size() / 4 > e->insts.count) more.resize(tw.tris.size() / 4 + tw.tris.size() / 16);
+  if (grown.ptr) {
     if (blas_u4)
       VT_CUDA(cudaMemcpyAsync(grown.ptr, e->nodes.ptr, blas_u4 * sizeof(uint4), cudaMemcpyDeviceToDevice, s));
     VT_CUDA(cudaStreamSynchronize(s));
     e->nodes = std::move(grown);
   }
+  if (more.ptr) e->insts = std::move(more);
   e->nodes_u4 = blas_u4 + tlas_u4;
   VT_CUDA(cudaMemcpyAsync(e->nodes.ptr + blas_u4, tw.nodes.data(), tw.nodes.size() * 4, cudaMemcpyHostToDevice, s));
   std::vector<float4> il(tw.tris.size() / 4), it(n * 4), ir(placed.rows.size() / 4);
   if (!il.empty()) std::memcpy(il.data(), tw.tris.data(), tw.tris.size() * 4);
   std::memcpy(it.data(), placed.recs.data(), n * sizeof(vt::InstanceRecord));
   if (!ir.empty()) std::memcpy(ir.data(), placed.rows.data(), placed.rows.size() * 4);
-  if (il.size() > e->insts.count) e->insts.resize(il.size() + il.size() / 4);
   if (!il.empty()) VT_CUDA(cudaMemcpyAsync(e->insts.ptr, il.data(), il.size() * sizeof(float4), cudaMemcpyHostToDevice, s));
   upload(e->inst_table, it, s);
   upload(e->inst_l2w, ir, s);
@@ -385,6 +387,7 @@ void update_instances(vt_engine* e, const vt_instance_desc* insts, size_t n, boo
   e->view.stack_depth = e->stack_depth;
   e->view.insts = e->insts.ptr;
   e->view.inst_table = e->inst_table.ptr;
+  if (insts != e->inst_descs.data()) e->inst_descs.assign(insts, insts + n);
   held.done = true;
   reset_accumulation(e);
   VT_CUDA(cudaStreamSynchronize(e->stream));
