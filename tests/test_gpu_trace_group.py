@@ -65,3 +65,42 @@ def test_material_flags(cuda):
         h, _ = e.trace_rays(r[a:a + n])
         assert np.array_equal(h.view(np.uint32), hits[a:a + n].view(np.uint32))
     e.dispose()
+
+
+@pytest.mark.parametrize("leaf", [1, 2, 4])
+@pytest.mark.parametrize("n", [16385, 16400, 20001, 70003])
+def test_occlusion_is_a_closest_hit(cuda, n, leaf):
+    """A large occlusion batch ends with eight lanes on each of a warp's last rays:
+    a segment is occluded just when the same ray has a closest hit -- long rays
+    through a loose soup, in leaves of 1 to 4, with warps that hold a few rays
+    only and with a trace order."""
+    soup = scenes.random_triangles(30000, seed=4)
+    rays = _rays(n, 11)
+    rays[::7, 3] = 0.0
+    rays[::7, 7] = 1e30
+    with vb.build_compressed_wide_bvh(soup.positions, soup.indices, maxLeafTriangles=leaf, traversalTree="reference") as g:
+        for order in (0, 3):
+            g.set_trace_order(order)
+            hit = g.intersect_first_hit(rays)["prim"] >= 0
+            occ = g.intersect_any_hit(rays)
+            assert 0 < hit.sum() < n
+            assert np.array_equal(occ.astype(bool), hit), (order, int((occ.astype(bool) != hit).sum()))
+
+
+@pytest.mark.parametrize("stage", [False, True])
+def test_shadow_flags_in_large_waves(cuda, stage):
+    """Two samples of 128 x 128 pixels in one wave of 32,768 paths or in two of
+    16,384 (eight lanes on every ray): the same image, bit for bit, with geometry
+    that casts no shadow."""
+    sc, cam = scenes.box_room(wall_cells=8, box_cells=4)
+    sc.materials[3].cast_shadow = False
+    imgs = []
+    for wave in (1 << 14, 1 << 15):
+        e = Engine(max_bounces=4, wave_paths=wave)
+        e.set_tuning(wave_paths=wave, stage_hot_nodes=stage)
+        e.set_scene(sc)
+        e.render_frame(cam, 128, 128, samples=2)
+        imgs.append(e.capture_frame())
+        e.dispose()
+    assert imgs[0].max() > 0
+    assert np.array_equal(imgs[0], imgs[1])
