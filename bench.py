@@ -727,7 +727,7 @@ def run_build(args, dev, local):
     out["query_soup_65536_tris"] = {"gpu_ms": round(g_ms[-1], 1), "host_ms": round(h_ms[-1], 1),
                                     "note": "the reference options' tree (4 per leaf, 16 bins) for export plus the "
                                             "traversal tree (2 per leaf, 32 bins, SAH-optimal 8-wide grouping), "
-                                            "incl. the publication proofs on the host copy"}
+                                            "incl. the publication proofs"}
     return out
 
 

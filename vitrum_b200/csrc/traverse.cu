@@ -1025,9 +1025,10 @@ template <bool ANY>
 void launch_trace_t(const TraceArgs& a, cudaStream_t s) {
   if (a.n == 0) return;
   // Up to here eight lanes per ray win (k_trace_group); measured, k_trace / group:
-  // closest hits of 1,000 rays on 4,096 triangles 49 / 35 us, 4,000 on 65,536
-  // 123 / 80, 16,000 in a room 75 / 51, 50,000 153 / 247; occlusion of 2,000 in the
-  // room 85 / 41, 30,000 95 / 60, 120,000 209 / 448
+  // closest hits of 1,000 rays on 4,096 loose triangles 49 / 35 us, 12,000 on 65,536
+  // 129 / 111, 16,384 137 / 139, 16,384 in a room of 16,384 75 / 64, 44,000 81 / 115;
+  // occlusion of 12,000 in a room of 262,146 118 / 58 (with finish_occlusion 81 / 71
+  // at 20,000), 36,000 in one of 16,384 51 / 59, on loose triangles 120 / 169
   constexpr size_t kGroupRays = 16384;
   if (!a.insts && a.n <= kGroupRays && !a.stage_nodes) {
     const int stk = std::min(std::max(a.stack_depth, 4), kMaxStack);
