@@ -38,7 +38,7 @@ enum : int { kColSh = 32, kColNormal = 48, kColRough = 51, kColDiffuse = 52, kCo
 
 // Query tiles in flight per inference CTA when the configuration leaves it open:
 // one CTA per SM keeps 4 T warps in flight; 1,048,576 queries of the 16 x 2^19
-// grid take 0.68 / 0.42 / 0.35 / 0.33 ms with T = 1 / 2 / 3 / 4.
+// grid take 0.67 / 0.41 / 0.34 / 0.31 ms with T = 1 / 2 / 3 / 4.
 constexpr int kDefaultInferTiles = 4;
 
 struct Config {

@@ -104,7 +104,7 @@ __device__ __forceinline__ Cell grid_cell(const View& v, int l, float3 n01) {
 // is 1, so the two rows differ in a few low bits, and 31 of 32 pairs fall into one
 // 128-byte line (7 of 8 into one 32-byte sector), which a warp's one access then
 // touches once instead of twice.  1,048,576 queries of the 16 x 2^19 grid, bound by
-// the L1's lookups: 383 -> 326 us.
+// the L1's lookups: 383 -> 326 us (312 with the layer inputs in TMEM, k_nrc_infer).
 struct PointPair {
   float3 even, odd;  // the even and the odd lane's point
   bool is_odd;       // this lane's place
@@ -269,6 +269,14 @@ __device__ __forceinline__ bool group_and(uint32_t id, bool p) {
 // columns each) and run independently -- each encodes its tile (16 levels x 8
 // table gathers per query), issues its own MMA chain from its first thread and
 // waits on its own mbarrier -- so one tile's gathers overlap another's MMAs.
+// The layer inputs are the MMAs' A operands in TMEM, written by the thread that owns
+// the row: shared memory holds the weights alone (50 KB instead of 66 to 114), and
+// what it gives up is L1 for the gathers that bound the kernel: 1,048,576 queries of
+// the 16 x 2^19 grid 326 -> 313 us.  (The coarsest level as a dense grid in shared
+// memory, beside 114 KB: 328; the two coarsest: 535, the L1 gone.)
+// TMEM columns of T tiles: 64 of accumulators and 32 of layer input each, rounded
+// up to a power of two
+__host__ __device__ constexpr uint32_t infer_cols(int t) { return t == 1 ? 128u : (t == 2 ? 256u : 512u); }
 template <int T>
 __global__ void __launch_bounds__(128 * T, T == 1 ? 3 : (T == 2 ? 2 : 1))
     k_nrc_infer(View v, const float4* __restrict__ recs, uint32_t stride, const uint32_t* __restrict__ n_dev,
@@ -277,12 +285,9 @@ __global__ void __launch_bounds__(128 * T, T == 1 ? 3 : (T == 2 ? 2 : 1))
   uint8_t* base = align1024(smem_raw);
   uint8_t* wt = base;
   const uint32_t tid = threadIdx.x & 127u, warp = tid >> 5, g = threadIdx.x >> 7, gid = g + 1;
-  // this warpgroup's tile: each layer's MMA has finished reading it before the
-  // epilogue writes the next layer's input over it
-  uint8_t* act = base + kLayers * kWBytes + g * kTileBytes;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(base + kLayers * kWBytes + T * kTileBytes) + g;
-  uint32_t* slot = reinterpret_cast<uint32_t*>(reinterpret_cast<uint64_t*>(base + kLayers * kWBytes + T * kTileBytes) + T);
-  constexpr uint32_t kCols = T == 1 ? 64u : (T == 2 ? 128u : 256u);  // a power of two >= 64 T
+  uint64_t* bar = reinterpret_cast<uint64_t*>(base + kLayers * kWBytes) + g;
+  uint32_t* slot = reinterpret_cast<uint32_t*>(reinterpret_cast<uint64_t*>(base + kLayers * kWBytes) + T);
+  constexpr uint32_t kCols = infer_cols(T);
   const uint32_t n = n_dev ? *n_dev : n_host;
   if ((uint32_t)blockIdx.x * T * kTile >= n) return;  // uniform per CTA: no tile, no TMEM
   if (threadIdx.x < 32) {
@@ -300,7 +305,10 @@ __global__ void __launch_bounds__(128 * T, T == 1 ? 3 : (T == 2 ? 2 : 1))
   tc::fence_after_sync();
   const uint32_t tmem = *slot + 64u * g;
   const uint32_t lane_addr = tmem + ((warp * 32u) << 16);
-  const uint32_t w_s = tc::smem_u32(wt), a_s = tc::smem_u32(act);
+  // this warpgroup's layer input, in TMEM (row = lane, 64 fp16 in 32 columns): each
+  // layer's MMA has finished reading it before the epilogue writes the next one over it
+  const uint32_t act = *slot + 64u * T + 32u * g, act_lane = act + ((warp * 32u) << 16);
+  const uint32_t w_s = tc::smem_u32(wt);
   uint32_t phase = 0;
   bool failed = false;
   for (uint32_t tile = blockIdx.x * T + g; tile * kTile < n && !failed; tile += gridDim.x * T) {
@@ -309,13 +317,16 @@ __global__ void __launch_bounds__(128 * T, T == 1 ? 3 : (T == 2 ? 2 : 1))
     uint32_t p[32];
     const float4* r = recs + (size_t)(valid ? i : 0) * stride;
     encode(v, __ldg(r), __ldg(r + 1), __ldg(r + 2), __ldg(r + 3), p);
-    store_row(act, tid, p);
-    tc::fence_async_smem();
+    tc::tmem_st32(act_lane, p);
+    tc::tmem_wait_st();
     tc::fence_before_sync();
     group_sync(gid);
     for (int l = 0; l < kLayers; ++l) {
       if (tid == 0) {
-        issue_fwd(tmem, a_s, w_s + l * kWBytes);
+        tc::fence_after_sync();
+#pragma unroll
+        for (uint32_t kk = 0; kk < 4; ++kk)
+          tc::mma_f16_ta(tmem, act + 8u * kk, tc::desc_k(w_s + l * kWBytes, kk), kIdesc, kk);
         tc::mma_commit(bar);
       }
       // thread-uniform bounded wait (per warpgroup); on failure `phase` keeps the pending parity
@@ -328,8 +339,8 @@ __global__ void __launch_bounds__(128 * T, T == 1 ? 3 : (T == 2 ? 2 : 1))
 #pragma unroll
         for (int k = 0; k < 32; ++k)
           p[k] = pack_h2(fmaxf(__uint_as_float(acc[2 * k]), 0.0f), fmaxf(__uint_as_float(acc[2 * k + 1]), 0.0f));
-        store_row(act, tid, p);
-        tc::fence_async_smem();
+        tc::tmem_st32(act_lane, p);
+        tc::tmem_wait_st();
         tc::fence_before_sync();
         group_sync(gid);
       } else {
@@ -684,7 +695,7 @@ __global__ void __launch_bounds__(256) k_nrc_adam(AdamPairs table, AdamPairs wei
                ibc1, ibc2, diag);
 }
 
-constexpr size_t infer_smem(int t) { return kLayers * kWBytes + (size_t)t * kTileBytes + 64 + 1024; }
+constexpr size_t kInferSmem = kLayers * kWBytes + 64 + 1024;
 constexpr size_t kTrainSmem = kLayers * kWBytes + (1 + kLayers) * kTileBytes + 64 + 1024;
 
 int sm_count() {
@@ -705,17 +716,17 @@ void launch_infer_t(const View& v, const float4* records, uint32_t rec_stride_f4
                     float* rgb_out, float4* radiance, cudaStream_t s) {
   static int per_sm = 0;
   if (!per_sm) {
-    cudaFuncSetAttribute(k_nrc_infer<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)infer_smem(T));
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_nrc_infer<T>, 128 * T, infer_smem(T));
-    // TMEM: 512 columns per SM, 64 T (rounded up to a power of two) per CTA
-    const int cols = T == 1 ? 64 : (T == 2 ? 128 : 256);
-    per_sm = per_sm < 512 / cols ? per_sm : 512 / cols;
+    cudaFuncSetAttribute(k_nrc_infer<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInferSmem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_nrc_infer<T>, 128 * T, kInferSmem);
+    // TMEM: 512 columns per SM
+    const int most = 512 / (int)infer_cols(T);
+    per_sm = per_sm < most ? per_sm : most;
     if (per_sm < 1) per_sm = 1;
   }
   const uint32_t tiles = (n + kTile - 1) / kTile;
   const uint32_t ctas = (tiles + T - 1) / T;
   const uint32_t cap = (uint32_t)(per_sm * sm_count());
-  k_nrc_infer<T><<<ctas < cap ? ctas : cap, 128 * T, infer_smem(T), s>>>(v, records, rec_stride_f4, n_dev, n, rgb_out,
+  k_nrc_infer<T><<<ctas < cap ? ctas : cap, 128 * T, kInferSmem, s>>>(v, records, rec_stride_f4, n_dev, n, rgb_out,
                                                                           radiance);
 }
 
@@ -726,10 +737,7 @@ void launch_infer(const View& v, const float4* records, uint32_t rec_stride_f4, 
   // (1,000 to 18,944 queries: 31 -> 17 us; 40,000: 33 -> 24 us)
   const uint32_t tiles = (n + kTile - 1) / kTile, sms = (uint32_t)sm_count();
   tiles_per_cta = (int)std::min<uint32_t>((uint32_t)tiles_per_cta, (tiles + sms - 1) / sms);
-  // tiles in flight per CTA: 1 to 4 (65 to 113 KB of shared memory).  Under the default
-  // carve-out one CTA runs per SM, which keeps most of the unified L1 for the hash-table gathers:
-  // asking for the largest shared-memory carve-out (three or two CTAs per SM) made two tiles per
-  // CTA slower (0.47 -> 0.82 ms for 1,048,576 queries), and so do five or six (0.335 against 0.326)
+  // tiles in flight per CTA: 1 to 4.  The registers and TMEM of four tiles fill an SM
   if (tiles_per_cta >= 4) launch_infer_t<4>(v, records, rec_stride_f4, n_dev, n, rgb_out, radiance, s);
   else if (tiles_per_cta == 3) launch_infer_t<3>(v, records, rec_stride_f4, n_dev, n, rgb_out, radiance, s);
   else if (tiles_per_cta == 2) launch_infer_t<2>(v, records, rec_stride_f4, n_dev, n, rgb_out, radiance, s);
