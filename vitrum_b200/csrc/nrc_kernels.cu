@@ -264,6 +264,10 @@ __device__ __forceinline__ bool group_and(uint32_t id, bool p) {
   return r != 0;
 }
 
+// TMEM columns of T tiles: 64 of accumulators and 32 of layer input each, rounded
+// up to a power of two
+__host__ __device__ constexpr uint32_t infer_cols(int t) { return t == 1 ? 128u : (t == 2 ? 256u : 512u); }
+
 // T tiles of 128 queries in flight per CTA, one per warpgroup (the MLP tile
 // knob): the warpgroups share the CTA's weight tiles and TMEM allocation (64
 // columns each) and run independently -- each encodes its tile (16 levels x 8
@@ -274,9 +278,6 @@ __device__ __forceinline__ bool group_and(uint32_t id, bool p) {
 // what it gives up is L1 for the gathers that bound the kernel: 1,048,576 queries of
 // the 16 x 2^19 grid 326 -> 313 us.  (The coarsest level as a dense grid in shared
 // memory, beside 114 KB: 328; the two coarsest: 535, the L1 gone.)
-// TMEM columns of T tiles: 64 of accumulators and 32 of layer input each, rounded
-// up to a power of two
-__host__ __device__ constexpr uint32_t infer_cols(int t) { return t == 1 ? 128u : (t == 2 ? 256u : 512u); }
 template <int T>
 __global__ void __launch_bounds__(128 * T, T == 1 ? 3 : (T == 2 ? 2 : 1))
     k_nrc_infer(View v, const float4* __restrict__ recs, uint32_t stride, const uint32_t* __restrict__ n_dev,
