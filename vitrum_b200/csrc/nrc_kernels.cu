@@ -53,12 +53,6 @@ __device__ __forceinline__ float2 unpack_h2(uint32_t u) {
   return __half22float2(h);
 }
 
-__device__ __forceinline__ void store_row(uint8_t* tile, uint32_t r, const uint32_t (&p)[32]) {
-#pragma unroll
-  for (int j = 0; j < 8; ++j)
-    *reinterpret_cast<uint4*>(tile + tc::sw128_offset(r, 8 * j)) = make_uint4(p[4 * j], p[4 * j + 1], p[4 * j + 2],
-                                                                               p[4 * j + 3]);
-}
 // normalised position in [0,1]^3 (normalizeToAabb, nrcEncoding.ts:166-178)
 __device__ __forceinline__ float3 normalise(const View& v, float px, float py, float pz) {
   return make_float3(fminf(1.0f, fmaxf(0.0f, (px - v.aabb_min[0]) * v.aabb_inv[0])),
