@@ -27,8 +27,9 @@
 // leaf's triangle offset is the start of its index range, which partitioning
 // never moves again.  Where no split beats a leaf the range is sorted by
 // (centroid on the widest axis, triangle index) and halved: by counting ranks
-// inside a subtree, by two stable device radix passes on a large node (rare:
-// the level waits for the host there).
+// inside a subtree, in one CTA's shared memory (k_sort) up to kSort triangles, by
+// two stable device radix passes above.  The level waits for the host there, which
+// launches the sorts: once a level, whatever the number of nodes.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -57,6 +58,14 @@ constexpr int kSmall = 256;
 constexpr int kSmallThreads = 256;
 constexpr int kChunk = 512;         // triangles of a large node per CTA
 constexpr int kChunkThreads = 256;
+// Nodes without a split of up to kSort triangles are sorted by one CTA each, side by
+// side: what fits the 48 KB of shared memory that need no opt-in.  262,144 triangles
+// of one centroid (1,023 nodes above kSmall in either tree) build in 27 ms, with
+// every one of those nodes sorted on the host's call in 164; 256 groups of 1,024 in
+// 5.5 instead of 110, as many spread triangles in 4.1.
+constexpr uint32_t kSort = 4096;
+constexpr int kSortThreads = 1024;
+constexpr size_t kSortSmem = (size_t)kSort * 12;
 constexpr uint32_t kFull = 0xFFFFFFFFu;
 
 using u64 = unsigned long long;
@@ -132,7 +141,8 @@ struct Ctl {
   uint32_t large[2], chunks[2]; // of a level, by its parity
   uint32_t bad;                 // input errors: 1 vertex out of range, 2 not finite; 4 capacity (never)
   uint32_t depth_error;
-  uint32_t stop;                // level + 1 whose large fallback sorts wait for the host
+  uint32_t stop;                // level + 1 whose fallback sorts wait for the host
+  uint32_t big;                 // one of them is above kSort
   uint32_t levels;              // levels of large nodes processed
   uint32_t max_depth;           // deepest node
   uint32_t total;               // nodes of the finished tree
@@ -501,7 +511,10 @@ __global__ void __launch_bounds__(128) k_choose(Work w, uint32_t level) {
           }
           w.nodes[l + i] = ch;
         }
-        if (s_decision == 3) ctl->stop = level + 1u;
+        if (s_decision == 3) {
+          ctl->stop = level + 1u;
+          if (count > kSort) ctl->big = 1u;
+        }
       }
     }
     s_carry = 0u;
@@ -614,12 +627,13 @@ __global__ void __launch_bounds__(kChunkThreads) k_scatter(Work w, uint32_t leve
   }
 }
 
-// Bounds of a node whose range was sorted on the host's call (ids: its index range).
-__global__ void __launch_bounds__(256) k_range_bounds(Work w, uint32_t node, const uint32_t* __restrict__ ids) {
-  LNode& N = w.nodes[node];
+// Bounds of a node whose range was sorted (ids: its index range), the part of the
+// threads first, first + step, ...; by whole warps.
+__device__ __forceinline__ void range_bounds(const Work& w, LNode& N, const uint32_t* ids, uint32_t first,
+                                             uint32_t step) {
   uint32_t mn[3] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, mx[3] = {0u, 0u, 0u};
   u64 cmn[3] = {~0ull, ~0ull, ~0ull}, cmx[3] = {0ull, 0ull, 0ull};
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < N.count; i += gridDim.x * blockDim.x) {
+  for (uint32_t i = first; i < N.count; i += step) {
     const uint4 l = w.boxes[2 * (size_t)ids[i]], h = w.boxes[2 * (size_t)ids[i] + 1];
     const uint32_t lo[3] = {l.x, l.y, l.z}, hi[3] = {h.x, h.y, h.z};
     for (int k = 0; k < 3; ++k) {
@@ -641,18 +655,64 @@ __global__ void __launch_bounds__(256) k_range_bounds(Work w, uint32_t node, con
     }
   }
 }
+__global__ void __launch_bounds__(256) k_range_bounds(Work w, uint32_t node, const uint32_t* __restrict__ ids) {
+  range_bounds(w, w.nodes[node], ids, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
 
-// Keys of the large fallback sort: -0 canonicalised to +0 (the reference's
-// comparator subtracts, so equal centroids tie and fall to the index), then
-// mapped to order-preserving integers.
+// Key of the fallback sort: -0 canonicalised to +0 (the reference's comparator
+// subtracts, so equal centroids tie and fall to the index), then mapped to an
+// order-preserving integer.
+__device__ __forceinline__ u64 sort_key(const uint4* boxes, uint32_t t, int axis) {
+  const uint4 l = boxes[2 * (size_t)t], h = boxes[2 * (size_t)t + 1];
+  double v = axis == 0 ? centroid(l.x, h.x) : (axis == 1 ? centroid(l.y, h.y) : centroid(l.z, h.z));
+  if (v == 0.0) v = 0.0;
+  return okey(v);
+}
 __global__ void k_sort_keys(const uint4* __restrict__ boxes, const uint32_t* __restrict__ ids, uint32_t c, int axis,
                             u64* __restrict__ keys) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= c) return;
-  const uint4 l = boxes[2 * (size_t)ids[i]], h = boxes[2 * (size_t)ids[i] + 1];
-  double v = axis == 0 ? centroid(l.x, h.x) : (axis == 1 ? centroid(l.y, h.y) : centroid(l.z, h.z));
-  if (v == 0.0) v = 0.0;
-  keys[i] = okey(v);
+  if (i < c) keys[i] = sort_key(boxes, ids[i], axis);
+}
+
+// A stopped level's nodes without a split of up to kSort triangles, one CTA each: a
+// bitonic sort of (key, triangle) pairs (all different) in shared memory, padded to
+// a power of two with pairs above every real one, then the children's bounds.
+__global__ void __launch_bounds__(kSortThreads) k_sort(Work w, uint32_t level) {
+  extern __shared__ __align__(16) unsigned char dyn[];
+  u64* key = reinterpret_cast<u64*>(dyn);
+  uint32_t* id = reinterpret_cast<uint32_t*>(dyn + 8 * (size_t)kSort);
+  const uint32_t p = level & 1u;
+  const LNode& N = w.nodes[w.list[p][blockIdx.x]];
+  const uint32_t count = N.count;
+  if (N.decision != 3 || count > kSort) return;
+  const uint32_t* src = w.idx[p] + N.begin;
+  uint32_t* dst = w.idx[p ^ 1u] + N.begin;
+  uint32_t m = 2;
+  while (m < count) m <<= 1;
+  for (uint32_t i = threadIdx.x; i < m; i += kSortThreads) {
+    id[i] = i < count ? src[i] : 0xFFFFFFFFu;
+    key[i] = i < count ? sort_key(w.boxes, id[i], N.axis) : ~0ull;
+  }
+  for (uint32_t k = 2; k <= m; k <<= 1)
+    for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+      __syncthreads();
+      for (uint32_t q = threadIdx.x; q < m / 2; q += kSortThreads) {
+        const uint32_t a = 2 * q - (q & (j - 1u)), b = a + j;
+        const u64 ka = key[a], kb = key[b];
+        const uint32_t ia = id[a], ib = id[b];
+        const bool above = ka > kb || (ka == kb && ia > ib);
+        if (above == ((a & k) == 0u)) {
+          key[a] = kb;
+          key[b] = ka;
+          id[a] = ib;
+          id[b] = ia;
+        }
+      }
+    }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < count; i += kSortThreads) dst[i] = id[i];
+  for (int i = 0; i < 2; ++i)
+    range_bounds(w, w.nodes[N.left + i], id + (i ? N.nl : 0u), threadIdx.x, kSortThreads);
 }
 
 // ---------------------------------------------------------------- small subtrees
@@ -1131,21 +1191,24 @@ BinaryBvhHost build_binary_gpu(const float* d_pos, size_t position_words, const 
       VT_CUDA(cudaGetLastError());
       read_ctl();
       if (ctl.stop) {
-        // the level's large fallback sorts, then its scatter, which waited with them
+        // the level's fallback sorts, then its scatter, which waited with them
         level = ctl.stop - 1u;
         const uint32_t p = level & 1u, n = ctl.large[p];
-        std::vector<uint32_t> ids(n);
-        VT_CUDA(cudaMemcpyAsync(ids.data(), w.list[p], n * 4, cudaMemcpyDeviceToHost, s));
-        VT_CUDA(cudaStreamSynchronize(s));
-        const uint32_t zero = 0;
-        VT_CUDA(cudaMemcpyAsync(&w.ctl->stop, &zero, sizeof zero, cudaMemcpyHostToDevice, s));
+        VT_CUDA(cudaMemsetAsync(&w.ctl->stop, 0, sizeof ctl.stop, s));
+        VT_CUDA(cudaMemsetAsync(&w.ctl->big, 0, sizeof ctl.big, s));
         k_scatter<<<w.max_chunks, kChunkThreads, 0, s>>>(w, level);
+        k_sort<<<n, kSortThreads, kSortSmem, s>>>(w, level);
         VT_CUDA(cudaGetLastError());
-        for (uint32_t id : ids) {
-          LNode N;
-          VT_CUDA(cudaMemcpyAsync(&N, w.nodes + id, sizeof N, cudaMemcpyDeviceToHost, s));
+        std::vector<LNode> nodes;  // the level's (they were made one after another)
+        if (ctl.big) {
+          const uint32_t first = level ? ctl.mark[level - 1] : 0u;
+          nodes.resize(ctl.mark[level] - first);
+          VT_CUDA(cudaMemcpyAsync(nodes.data(), w.nodes + first, nodes.size() * sizeof(LNode), cudaMemcpyDeviceToHost,
+                                  s));
           VT_CUDA(cudaStreamSynchronize(s));
-          if (N.decision != 3) continue;
+        }
+        for (const LNode& N : nodes) {
+          if (N.decision != 3 || N.count <= kSort) continue;
           uint32_t* dst = w.idx[p ^ 1u] + N.begin;
           sort_range(w.boxes, w.idx[p] + N.begin, dst, N.count, N.axis, s);
           for (int i = 0; i < 2; ++i) {
