@@ -600,7 +600,8 @@ vt_status vt_update_instances(vt_engine* engine, const vt_instance_desc* instanc
  * instances.  Its bottom-level tree is rebuilt and spliced in place (later
  * meshes rebased when its size changed), then the top level is refitted over
  * the instances' new bounds, or rebuilt when `rebuild` is 1.  The other meshes'
- * trees are untouched; accumulation restarts.  A scene without instances has
+ * trees are untouched; accumulation restarts.  An update that fails (out of
+ * memory included) leaves the scene as it was.  A scene without instances has
  * one flat tree: VT_ERR_STATE (set the scene again). */
 vt_status vt_update_mesh(vt_engine* engine, size_t mesh_index, const vt_mesh_desc* mesh, int32_t rebuild);
 

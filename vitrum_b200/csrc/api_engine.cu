@@ -65,6 +65,7 @@ struct vt_engine {
   vt::PoolBuffer<uint4> nodes;
   size_t nodes_u4 = 0;             // words in use (an instance update may leave room behind them)
   vt::PoolBuffer<float4> tris;
+  size_t tris_f4 = 0;              // likewise, of a mesh update
   int wide_depth = 1;
   int stack_depth = 16;            // traversal stack entries the scene needs
   DeviceBuffer<float4> insts;      // instance records in top-level leaf order
@@ -241,6 +242,7 @@ void set_scene(vt_engine* e, const vt_scene_desc* sc) {
   e->nodes = std::move(n.nodes);
   e->nodes_u4 = n_u4;
   e->tris = std::move(n.tris);
+  e->tris_f4 = e->tris.count;
   e->insts = std::move(n.insts);
   e->inst_table = std::move(n.inst_table);
   e->inst_l2w = std::move(n.inst_l2w);
@@ -316,6 +318,90 @@ void set_scene(vt_engine* e, const vt_scene_desc* sc) {
   VT_CUDA(cudaStreamSynchronize(e->stream));
 }
 
+// The top level of a two-level scene over given placements and bottom levels.
+struct TopLevel {
+  vt::BinaryBvhHost tree;
+  vt::WideBvhHost wide;                    // its nodes follow the bottom levels', from tlas_root on
+  std::vector<float4> insts, table, rows;  // instance records in leaf order, by instance; local-to-world rows
+};
+
+TopLevel plan_top_level(const vt_engine* e, const vt_instance_desc* insts, size_t n, bool rebuild,
+                        const std::vector<uint32_t>& blas_root,
+                        const std::vector<std::array<double, 6>>& local_box, uint32_t tlas_root) {
+  const vt::InstanceSet placed = vt::place_instances(insts, n, e->mats_host, blas_root, local_box);
+  const vt::SceneBuild sb = scene_build_of(e);
+  TopLevel t;
+  if (rebuild) {
+    t.tree = vt::build_top_level(sb, placed.aabbs.data(), n);
+  } else {
+    t.tree = e->binary;
+    vt::refit_tlas_host(t.tree, placed.aabbs.data(), n);
+  }
+  t.wide = vt::encode_top_level(sb, t.tree, placed.recs, tlas_root);
+  t.insts.resize(t.wide.tris.size() / 4);
+  t.table.resize(n * 4);
+  t.rows.resize(placed.rows.size() / 4);
+  if (!t.insts.empty()) std::memcpy(t.insts.data(), t.wide.tris.data(), t.wide.tris.size() * 4);
+  std::memcpy(t.table.data(), placed.recs.data(), n * sizeof(vt::InstanceRecord));
+  if (!t.rows.empty()) std::memcpy(t.rows.data(), placed.rows.data(), placed.rows.size() * 4);
+  return t;
+}
+
+// Larger arrays for a scene update, where the present ones do not hold it (empty:
+// they do).  An update allocates all of them before it replaces or overwrites
+// anything, so that one which runs out of memory leaves the scene as it was.
+struct UpdateRoom {
+  vt::PoolBuffer<uint4> nodes;
+  vt::PoolBuffer<float4> tris;
+  DeviceBuffer<float4> insts;
+};
+
+UpdateRoom make_room(vt_engine* e, const TopLevel& t, uint32_t tlas_root, size_t tris_f4) {
+  UpdateRoom room;
+  const size_t blas_u4 = (size_t)tlas_root * 5, tlas_u4 = t.wide.nodes.size() / 4;
+  if (blas_u4 + tlas_u4 > e->nodes.count) room.nodes.resize(blas_u4 + tlas_u4 + tlas_u4 / 4, e->stream);
+  if (tris_f4 > e->tris.count) room.tris.resize(tris_f4, e->stream);
+  if (t.insts.size() > e->insts.count) room.insts.resize(t.insts.size() + t.insts.size() / 4);
+  return room;
+}
+
+// Writes the update's arrays and takes them over; with spliced, the bottom levels
+// and triangle records too, from the engine's host copies.  Nothing here allocates.
+void commit_update(vt_engine* e, TopLevel&& t, UpdateRoom&& room, uint32_t tlas_root, bool spliced) {
+  cudaStream_t s = e->stream;
+  uint4* nodes = room.nodes.ptr ? room.nodes.ptr : e->nodes.ptr;
+  float4* insts = room.insts.ptr ? room.insts.ptr : e->insts.ptr;
+  const size_t blas_u4 = (size_t)tlas_root * 5, tlas_u4 = t.wide.nodes.size() / 4;
+  if (spliced) {
+    float4* tris = room.tris.ptr ? room.tris.ptr : e->tris.ptr;
+    VT_CUDA(cudaMemcpyAsync(nodes, e->blas_words.data(), e->blas_words.size() * 4, cudaMemcpyHostToDevice, s));
+    VT_CUDA(cudaMemcpyAsync(tris, e->rec_host.data(), e->rec_host.size() * 4, cudaMemcpyHostToDevice, s));
+    e->tris_f4 = std::max<size_t>(e->rec_host.size() / 4, 1);
+  } else if (room.nodes.ptr && blas_u4) {
+    VT_CUDA(cudaMemcpyAsync(nodes, e->nodes.ptr, blas_u4 * sizeof(uint4), cudaMemcpyDeviceToDevice, s));
+  }
+  VT_CUDA(cudaMemcpyAsync(nodes + blas_u4, t.wide.nodes.data(), t.wide.nodes.size() * 4, cudaMemcpyHostToDevice, s));
+  if (!t.insts.empty())
+    VT_CUDA(cudaMemcpyAsync(insts, t.insts.data(), t.insts.size() * sizeof(float4), cudaMemcpyHostToDevice, s));
+  upload(e->inst_table, t.table, s);  // (one entry per instance: never another size)
+  upload(e->inst_l2w, t.rows, s);
+  VT_CUDA(cudaStreamSynchronize(s));
+  if (room.nodes.ptr) e->nodes = std::move(room.nodes);
+  if (room.tris.ptr) e->tris = std::move(room.tris);
+  if (room.insts.ptr) e->insts = std::move(room.insts);
+  e->nodes_u4 = blas_u4 + tlas_u4;
+  e->tlas_root = tlas_root;
+  e->binary = std::move(t.tree);
+  e->wide_depth = t.wide.depth + e->blas_depth;
+  e->stack_depth = std::max(e->stack_depth, 2 * e->wide_depth + 6);
+  e->view.nodes = e->nodes.ptr;
+  e->view.tris = e->tris.ptr;
+  e->view.root = tlas_root;
+  e->view.stack_depth = e->stack_depth;
+  e->view.insts = e->insts.ptr;
+  e->view.inst_table = e->inst_table.ptr;
+}
+
 // New placements for the instances of a two-level scene (refitTlasTransforms /
 // rebuildTlasReuseBlas, shared-bvh/src/scenePack.ts:1310, 1635): the bottom
 // levels stay; the top level is refitted (same topology, new bounds) or rebuilt
@@ -326,18 +412,8 @@ void update_instances(vt_engine* e, const vt_instance_desc* insts, size_t n, boo
     fail(VT_ERR_INVALID_ARGUMENT, "expected " + std::to_string(e->n_instances) + " instances, got " +
                                       std::to_string(n) + " (set a new scene to change the membership)");
   if (!insts) fail(VT_ERR_INVALID_ARGUMENT, "instances is null");
-  vt::InstanceSet placed = vt::place_instances(insts, n, e->mats_host, e->blas_root, e->local_box);
-  vt::BinaryBvhHost tl;
-  const vt::SceneBuild sb = scene_build_of(e);
-  if (rebuild) {
-    tl = vt::build_top_level(sb, placed.aabbs.data(), n);
-  } else {
-    tl = e->binary;
-    vt::refit_tlas_host(tl, placed.aabbs.data(), n);
-  }
-  vt::WideBvhHost tw = vt::encode_top_level(sb, tl, placed.recs, e->tlas_root);
-  cudaStream_t s = e->stream;
-  VT_CUDA(cudaStreamSynchronize(s));
+  TopLevel t = plan_top_level(e, insts, n, rebuild, e->blas_root, e->local_box, e->tlas_root);
+  VT_CUDA(cudaStreamSynchronize(e->stream));
   // The captured graphs hold these pointers, the stack bound and, where nodes are
   // staged or queues traced in spatial order, the node count and the scene's
   // bounds.  They stay while those do: arrays grow with room behind them and the
@@ -357,37 +433,8 @@ void update_instances(vt_engine* e, const vt_instance_desc* insts, size_t n, boo
         e->drop_graphs();
     }
   } held{e, e->nodes.ptr, e->insts.ptr, e->inst_table.ptr, e->nodes_u4, e->stack_depth};
-  const size_t blas_u4 = (size_t)e->tlas_root * 5, tlas_u4 = tw.nodes.size() / 4;
-  // both arrays before either is replaced: an update that runs out of memory leaves the scene as it was
-  vt::PoolBuffer<uint4> grown;
-  DeviceBuffer<float4> more;
-  if (blas_u4 + tlas_u4 > e->nodes.count) grown.resize(blas_u4 + tlas_u4 + tlas_u4 / 4, s);
-  if (tw.tris.size() / 4 > e->insts.count) more.resize(tw.tris.size() / 4 + tw.tris.size() / 16);
-  if (grown.ptr) {
-    if (blas_u4)
-      VT_CUDA(cudaMemcpyAsync(grown.ptr, e->nodes.ptr, blas_u4 * sizeof(uint4), cudaMemcpyDeviceToDevice, s));
-    VT_CUDA(cudaStreamSynchronize(s));
-    e->nodes = std::move(grown);
-  }
-  if (more.ptr) e->insts = std::move(more);
-  e->nodes_u4 = blas_u4 + tlas_u4;
-  VT_CUDA(cudaMemcpyAsync(e->nodes.ptr + blas_u4, tw.nodes.data(), tw.nodes.size() * 4, cudaMemcpyHostToDevice, s));
-  std::vector<float4> il(tw.tris.size() / 4), it(n * 4), ir(placed.rows.size() / 4);
-  if (!il.empty()) std::memcpy(il.data(), tw.tris.data(), tw.tris.size() * 4);
-  std::memcpy(it.data(), placed.recs.data(), n * sizeof(vt::InstanceRecord));
-  if (!ir.empty()) std::memcpy(ir.data(), placed.rows.data(), placed.rows.size() * 4);
-  if (!il.empty()) VT_CUDA(cudaMemcpyAsync(e->insts.ptr, il.data(), il.size() * sizeof(float4), cudaMemcpyHostToDevice, s));
-  upload(e->inst_table, it, s);
-  upload(e->inst_l2w, ir, s);
-  VT_CUDA(cudaStreamSynchronize(s));
-  e->binary = std::move(tl);
-  e->wide_depth = tw.depth + e->blas_depth;
-  e->stack_depth = std::max(e->stack_depth, 2 * e->wide_depth + 6);
-  e->view.nodes = e->nodes.ptr;
-  e->view.stack_depth = e->stack_depth;
-  e->view.insts = e->insts.ptr;
-  e->view.inst_table = e->inst_table.ptr;
-  if (insts != e->inst_descs.data()) e->inst_descs.assign(insts, insts + n);
+  commit_update(e, std::move(t), make_room(e, t, e->tlas_root, 0), e->tlas_root, false);
+  e->inst_descs.assign(insts, insts + n);
   held.done = true;
   reset_accumulation(e);
   VT_CUDA(cudaStreamSynchronize(e->stream));
@@ -398,7 +445,8 @@ void update_instances(vt_engine* e, const vt_instance_desc* insts, size_t n, boo
 // :1006-1100): the mesh's bottom level is rebuilt and spliced into the
 // concatenated node and record arrays; when its size changed, the later
 // meshes' node and record indices and roots are rebased.  The top level is
-// then refitted (or rebuilt) over the instances' new bounds.
+// refitted (or rebuilt) over the instances' new bounds.  Like the other updates
+// it builds and allocates everything first: a failure leaves the scene as it was.
 void update_mesh(vt_engine* e, size_t m, const vt_mesh_desc* md, bool rebuild) {
   if (!e->has_scene || e->n_instances == 0)
     fail(VT_ERR_STATE, "mesh updates need a scene with instances (set the scene again to change a flat scene)");
@@ -411,13 +459,29 @@ void update_mesh(vt_engine* e, size_t m, const vt_mesh_desc* md, bool rebuild) {
   const uint32_t node0 = e->blas_root[m], rec0 = e->blas_rec_start[m];
   const uint32_t node1 = m + 1 < nm ? e->blas_root[m + 1] : e->tlas_root;
   const uint32_t rec1 = m + 1 < nm ? e->blas_rec_start[m + 1] : (uint32_t)(e->rec_host.size() / 16);
-  const uint32_t old_tlas_root = e->tlas_root;
   vt::BlasPack bp = vt::pack_blas(pos, idx, md->material, node0, rec0, e->opts.bvh_max_leaf, scene_build_of(e));
   const int64_t dn = (int64_t)(bp.wide.nodes.size() / 20) - (int64_t)(node1 - node0);
   const int64_t dr = (int64_t)(bp.wide.tris.size() / 16) - (int64_t)(rec1 - rec0);
   if ((int64_t)e->rec_host.size() / 16 + dr + 32 >= (int64_t)0x40000000)
     fail(VT_ERR_RANGE, "triangle records exceed 2^30");
-  // splice, then rebase the later bottom levels (child base at word 4, triangle base at word 5)
+  // where everything will lie
+  std::vector<uint32_t> blas_root = e->blas_root, rec_start = e->blas_rec_start;
+  std::vector<std::array<double, 6>> local_box = e->local_box;
+  for (size_t k = m + 1; k < nm; ++k) {
+    blas_root[k] = (uint32_t)((int64_t)blas_root[k] + dn);
+    rec_start[k] = (uint32_t)((int64_t)rec_start[k] + dr);
+  }
+  local_box[m] = bp.local_box;
+  const uint32_t tlas_root = (uint32_t)((int64_t)e->tlas_root + dn);
+  TopLevel t = plan_top_level(e, e->inst_descs.data(), e->inst_descs.size(), rebuild, blas_root, local_box, tlas_root);
+  VT_CUDA(cudaStreamSynchronize(e->stream));
+  const size_t rec_words = (size_t)((int64_t)e->rec_host.size() + 16 * dr);
+  UpdateRoom room = make_room(e, t, tlas_root, std::max<size_t>(rec_words / 4, 1));
+  e->blas_words.reserve((size_t)tlas_root * 20);
+  e->rec_host.reserve(rec_words);
+  // nothing below allocates: splice, then rebase the later bottom levels (child base
+  // at word 4, triangle base at word 5)
+  e->drop_graphs();
   e->blas_words.erase(e->blas_words.begin() + (size_t)node0 * 20, e->blas_words.begin() + (size_t)node1 * 20);
   e->blas_words.insert(e->blas_words.begin() + (size_t)node0 * 20, bp.wide.nodes.begin(), bp.wide.nodes.end());
   e->rec_host.erase(e->rec_host.begin() + (size_t)rec0 * 16, e->rec_host.begin() + (size_t)rec1 * 16);
@@ -428,33 +492,17 @@ void update_mesh(vt_engine* e, size_t m, const vt_mesh_desc* md, bool rebuild) {
       e->blas_words[20 * w + 4] = (uint32_t)((int64_t)e->blas_words[20 * w + 4] + dn);
       e->blas_words[20 * w + 5] = (uint32_t)((int64_t)e->blas_words[20 * w + 5] + dr);
     }
-    for (size_t k = m + 1; k < nm; ++k) {
-      e->blas_root[k] = (uint32_t)((int64_t)e->blas_root[k] + dn);
-      e->blas_rec_start[k] = (uint32_t)((int64_t)e->blas_rec_start[k] + dr);
-    }
   }
-  e->tlas_root = (uint32_t)((int64_t)e->tlas_root + dn);
-  e->local_box[m] = bp.local_box;
+  e->blas_root = std::move(blas_root);
+  e->blas_rec_start = std::move(rec_start);
+  e->local_box = std::move(local_box);
   e->blas_depths[m] = bp.wide.depth;
   e->blas_depth = *std::max_element(e->blas_depths.begin(), e->blas_depths.end());
   e->ntri += (int64_t)md->triangle_count - (int64_t)e->mesh_tris[m];
   e->mesh_tris[m] = md->triangle_count;
-  const size_t tlas_u4 = e->nodes_u4 - (size_t)old_tlas_root * 5;
-  // upload the bottom levels and records; the top level follows in update_instances
-  cudaStream_t s = e->stream;
-  VT_CUDA(cudaStreamSynchronize(s));
-  e->drop_graphs();
-  const size_t blas_u4 = e->blas_words.size() / 4;
-  e->nodes_u4 = blas_u4 + tlas_u4;
-  e->nodes.resize(e->nodes_u4, s);  // the top level's part is written by update_instances
-  VT_CUDA(cudaMemcpyAsync(e->nodes.ptr, e->blas_words.data(), e->blas_words.size() * 4, cudaMemcpyHostToDevice, s));
-  e->tris.resize(std::max<size_t>(e->rec_host.size() / 4, 1), s);
-  VT_CUDA(cudaMemcpyAsync(e->tris.ptr, e->rec_host.data(), e->rec_host.size() * 4, cudaMemcpyHostToDevice, s));
-  VT_CUDA(cudaStreamSynchronize(s));
-  e->view.tris = e->tris.ptr;
-  e->view.root = e->tlas_root;
-  const std::vector<vt_instance_desc> insts = e->inst_descs;
-  update_instances(e, insts.data(), insts.size(), rebuild);
+  commit_update(e, std::move(t), std::move(room), tlas_root, true);
+  reset_accumulation(e);
+  VT_CUDA(cudaStreamSynchronize(e->stream));
 }
 
 // ---------------------------------------------------------------- waves
@@ -1300,7 +1348,7 @@ vt_status vt_engine_export_scene(const vt_engine* e, uint32_t* node_words, size_
     if (!e) fail(VT_ERR_INVALID_ARGUMENT, "engine is null");
     if (!e->has_scene) fail(VT_ERR_STATE, "export before setScene");
     vt::DeviceScope ds(e->device);
-    const size_t nw = e->nodes_u4 * 4, nf = e->tris.count * 4;
+    const size_t nw = e->nodes_u4 * 4, nf = e->tris_f4 * 4;
     if (out_words) *out_words = nw;
     if (out_floats) *out_floats = nf;
     VT_CUDA(cudaStreamSynchronize(e->stream));
