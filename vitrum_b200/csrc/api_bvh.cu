@@ -36,6 +36,11 @@ void configure_scratch_pool() {
     unsigned long long keep = 1ull << 30;
     cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
   }
+  // Eight bytes of each device stay allocated, and with them the driver's smallest
+  // unit of mapped memory: wait_as_free_does takes 7 us next to them and maps and
+  // unmaps that unit without, 575 us.
+  void* stays = nullptr;
+  if (cudaMalloc(&stays, 8) != cudaSuccess) cudaGetLastError();
   done[dev] = true;
 }
 
@@ -90,10 +95,7 @@ static void publish(vt_bvh* b, const uint32_t* words, size_t n_nodes, const floa
     VT_CUDA(cudaMemsetAsync(b->status.ptr, 0, sizeof(int), s));
     VT_CUDA(cudaStreamSynchronize(s));
   } catch (...) {
-    b->nodes.release();  // here, on the device they belong to
-    b->tris.release();
-    b->status.release();
-    b->counter.release();
+    b->release_arrays();  // here, on the device they belong to
     throw;
   }
   b->wide_count = (int64_t)n_nodes;

@@ -18,6 +18,7 @@ struct vt_bvh {
   vt::PoolBuffer<float4> tris;           // triangle records (at least one allocated)
   vt::PoolBuffer<int> status;            // traversal status word
   vt::PoolBuffer<unsigned long long> counter;  // persistent-kernel ray counter (calls on one bvh are serialised)
+  void release_arrays() { vt::PoolBuffer<int>::release_all(nodes, tris, status, counter); }
   int64_t ntri = 0;
   int64_t wide_count = 0;                // 8-wide nodes
   int64_t rec_count = 0;                 // triangle records
@@ -36,6 +37,7 @@ struct vt_bvh {
   int order_bits = 0;
   vt::DeviceBuffer<uint32_t> order_keys, order_idx, order_counts;
   ~vt_bvh() {
+    release_arrays();
     for (cudaStream_t& s : copy_streams)
       if (s) cudaStreamDestroy(s);
   }

@@ -141,12 +141,25 @@ struct ScratchBuffer {
   size_t bytes() const { return count * sizeof(T); }
 };
 
+// Waits until no work is left on the current device, as the release of a cudaMalloc
+// block does: by releasing one (7 us with its allocation).  cudaDeviceSynchronize is
+// no substitute: while any thread captures a stream of the device it fails, and that
+// capture fails with it.  False: the wait did not happen (this thread is capturing).
+inline bool wait_as_free_does() {
+  void* block = nullptr;
+  const cudaError_t e = cudaMalloc(&block, 8);
+  if (e == cudaSuccess) return cudaFree(block) == cudaSuccess;
+  cudaGetLastError();
+  return e == cudaErrorMemoryAllocation && cudaDeviceSynchronize() == cudaSuccess;
+}
+
 // Owning device memory from the same pool, for arrays that outlive the call
 // that fills them (trees, scenes): allocated in the order of stream s (other
-// streams may use it once s has been synchronised), released like cudaFree, when
-// no work is left on the device.  A tree built, used and dropped every frame
-// takes microseconds here where cudaMalloc and cudaFree took 1-2 ms and, now and
-// then, tens.
+// streams may use it once s has been synchronised), released as DeviceBuffer is,
+// when no work is left on the device; where cudaFree would fail (see above) it is
+// left allocated, as there.  A tree built, used and dropped every frame takes
+// microseconds here where cudaMalloc and cudaFree took 1-2 ms and, now and then,
+// tens.
 template <class T>
 struct PoolBuffer {
   T* ptr = nullptr;
@@ -160,13 +173,14 @@ struct PoolBuffer {
     return *this;
   }
   ~PoolBuffer() { release(); }
-  void release() {
-    if (ptr) {
-      cudaDeviceSynchronize();
-      cudaFreeAsync(ptr, nullptr);
-    }
-    ptr = nullptr;
-    count = 0;
+  void release() { release_all(*this); }
+  // Several buffers of one device behind one wait.
+  template <class... B>
+  static void release_all(B&... b) {
+    const bool idle = ((b.ptr != nullptr) || ...) && wait_as_free_does();
+    // (cudaFree of pool memory returns it to the pool at once, without a wait of its own)
+    ((idle && b.ptr ? (void)cudaFree(b.ptr) : (void)0), ...);
+    ((b.ptr = nullptr, b.count = 0), ...);
   }
   void resize(size_t n, cudaStream_t s) {
     if (n == count) return;
