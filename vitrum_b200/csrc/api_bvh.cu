@@ -27,21 +27,21 @@ void set_last_error(const std::string& msg) { t_last_error = msg; }
 void clear_last_error() { t_last_error.clear(); }
 
 void configure_scratch_pool() {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return;
-  static bool done[64] = {};
-  if (dev < 0 || dev >= 64 || done[dev]) return;
-  cudaMemPool_t pool;
-  if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
-    unsigned long long keep = 1ull << 30;
-    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-  }
-  // Eight bytes of each device stay allocated, and with them the driver's smallest
-  // unit of mapped memory: wait_as_free_does takes 7 us next to them and maps and
-  // unmaps that unit without, 575 us.
-  void* stays = nullptr;
-  if (cudaMalloc(&stays, 8) != cudaSuccess) cudaGetLastError();
-  done[dev] = true;
+  static PerDevice<bool> configured;
+  const int dev = current_device();
+  configured.get(dev, [dev] {
+    cudaMemPool_t pool;
+    if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
+      unsigned long long keep = 1ull << 30;
+      cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    }
+    // Eight bytes of each device stay allocated, and with them the driver's smallest
+    // unit of mapped memory: wait_as_free_does takes 7 us next to them and maps and
+    // unmaps that unit without, 575 us.
+    void* stays = nullptr;
+    if (cudaMalloc(&stays, 8) != cudaSuccess) cudaGetLastError();
+    return true;
+  });
 }
 
 thread_local long long t_alloc_fail_countdown = 0;  // 0: disarmed

@@ -1152,12 +1152,12 @@ BinaryBvhHost build_binary_gpu(const float* d_pos, size_t position_words, const 
   ScratchBuffer<uint32_t> order(ntri, s);
   ScratchBuffer<BinaryNode> dout(2 * ntri, s);
   const size_t small_smem = sizeof(Small) + (size_t)(kSmallThreads / 32) * 14 * o.bins * 4;
-  static bool attr = false;
-  if (!attr) {
+  static PerDevice<bool> opted_in;
+  opted_in.get(current_device(), [] {
     VT_CUDA(cudaFuncSetAttribute(k_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(sizeof(Small) + (size_t)(kSmallThreads / 32) * 14 * kMaxBins * 4)));
-    attr = true;
-  }
+    return true;
+  });
   const uint32_t init = std::max<uint32_t>({1u, (uint32_t)((ntri + kChunk - 1) / kChunk), (uint32_t)(21 * o.bins)});
   k_init<<<(init + 255) / 256, 256, 0, s>>>(w);
   VT_CUDA(cudaGetLastError());

@@ -26,6 +26,7 @@
 
 #include "nrc.h"
 #include "tc_sm100.cuh"
+#include "vt_common.h"
 
 namespace vt {
 namespace nrc {
@@ -709,15 +710,13 @@ void level_resolutions(const Config& c, float* out) {
 template <int T>
 void launch_infer_t(const View& v, const float4* records, uint32_t rec_stride_f4, const uint32_t* n_dev, uint32_t n,
                     float* rgb_out, float4* radiance, cudaStream_t s) {
-  static int per_sm = 0;
-  if (!per_sm) {
-    cudaFuncSetAttribute(k_nrc_infer<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInferSmem);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_nrc_infer<T>, 128 * T, kInferSmem);
-    // TMEM: 512 columns per SM
-    const int most = 512 / (int)infer_cols(T);
-    per_sm = per_sm < most ? per_sm : most;
-    if (per_sm < 1) per_sm = 1;
-  }
+  static PerDevice<int> resident;
+  const int per_sm = resident.get(current_device(), [] {
+    int ctas = 0;
+    VT_CUDA(cudaFuncSetAttribute(k_nrc_infer<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInferSmem));
+    VT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, k_nrc_infer<T>, 128 * T, kInferSmem));
+    return std::max(1, std::min(ctas, 512 / (int)infer_cols(T)));  // TMEM: 512 columns per SM
+  });
   const uint32_t tiles = (n + kTile - 1) / kTile;
   const uint32_t ctas = (tiles + T - 1) / T;
   const uint32_t cap = (uint32_t)(per_sm * sm_count());
@@ -741,11 +740,11 @@ void launch_infer(const View& v, const float4* records, uint32_t rec_stride_f4, 
 
 void launch_train(const View& v, const float4* samples, uint32_t n, cudaStream_t s) {
   if (n == 0) return;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_nrc_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrainSmem);
-    attr = true;
-  }
+  static PerDevice<bool> opted_in;
+  opted_in.get(current_device(), [] {
+    VT_CUDA(cudaFuncSetAttribute(k_nrc_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrainSmem));
+    return true;
+  });
   const uint32_t tiles = (n + kTile - 1) / kTile;
   const uint32_t grid = tiles < (uint32_t)sm_count() ? tiles : (uint32_t)sm_count();
   k_nrc_train<<<grid, 128 * kTrainGroups, kTrainSmem, s>>>(v, samples, n);

@@ -11,6 +11,7 @@
 #include <string>
 
 #include "../../include/vitrum_pt.h"
+#include "per_device.h"
 
 namespace vt {
 
@@ -32,6 +33,12 @@ inline void cuda_check(cudaError_t e, const char* what) {
   }
 }
 #define VT_CUDA(call) ::vt::cuda_check((call), #call)
+
+inline int current_device() {
+  int device = 0;
+  VT_CUDA(cudaGetDevice(&device));
+  return device;
+}
 
 // Runs `fn` and converts exceptions into a vt_status plus thread-local message.
 template <class F>
