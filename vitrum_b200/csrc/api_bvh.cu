@@ -184,6 +184,23 @@ static void order_batch(vt_bvh* b, TraceArgs& a, size_t off, int k, cudaStream_t
   a.order = o.order;
 }
 
+// Device memory nothing writes any more to the host, on a stream of its own and with
+// this thread's capture restrictions set aside: a call like this one, which needs
+// nothing of the caller's streams, stays open while one of them is being captured.
+static void read_back(void* to, const void* from, size_t bytes) {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  VT_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+  cudaStream_t s = nullptr;
+  cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+  if (e == cudaSuccess) {
+    e = cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    cudaStreamDestroy(s);
+  }
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  VT_CUDA(e);
+}
+
 static void check_status(vt_bvh* b) {
   int st = 0;
   VT_CUDA(cudaMemcpy(&st, b->status.ptr, sizeof(int), cudaMemcpyDeviceToHost));
@@ -267,11 +284,11 @@ vt_status vt_bvh_export_wide(const vt_bvh* b, uint32_t* node_words, size_t word_
     DeviceScope ds(b->device);
     if (node_words) {
       if (word_capacity < nw) fail(VT_ERR_RANGE, "node buffer too small");
-      VT_CUDA(cudaMemcpy(node_words, b->nodes.ptr, nw * 4, cudaMemcpyDeviceToHost));
+      read_back(node_words, b->nodes.ptr, nw * 4);
     }
     if (records) {
       if (float_capacity < nf) fail(VT_ERR_RANGE, "record buffer too small");
-      if (nf) VT_CUDA(cudaMemcpy(records, b->tris.ptr, nf * 4, cudaMemcpyDeviceToHost));
+      if (nf) read_back(records, b->tris.ptr, nf * 4);
     }
   });
 }
