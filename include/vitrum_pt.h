@@ -663,6 +663,18 @@ vt_status vt_engine_set_wait_limit(vt_engine* engine, int64_t cycles);
  */
 vt_status vt_debug_fail_device_allocation(int64_t nth);
 
+/*
+ * Test hook: the publication proofs over given words, on_device 1 as device
+ * builds run them (on the current device), 0 as host builds do.  Binary nodes
+ * are 8 words each and lie over triangle_count triangles (NULL: skipped); wide
+ * nodes are 20 words, triangle records 16 floats each (NULL: skipped).
+ * VT_ERR_BUILD where a proof does not hold or a traversal would need more than
+ * stack_capacity entries.  The words are only read; no ray is traced.
+ */
+vt_status vt_debug_prove_bvh(int32_t on_device, const uint32_t* binary_words, size_t binary_nodes,
+                             const uint32_t* wide_words, size_t wide_nodes, const float* records,
+                             size_t record_count, size_t triangle_count, int32_t stack_capacity);
+
 vt_status vt_reset(vt_engine* engine);
 vt_status vt_engine_get_stats(const vt_engine* engine, vt_engine_stats* out_stats);
 /* Engine.dispose */

@@ -128,6 +128,7 @@ SIGNATURES = {
     "vt_nrc_train_device": [P, P, SZ, P],
     "vt_engine_set_wait_limit": [P, ctypes.c_int64],
     "vt_debug_fail_device_allocation": [ctypes.c_int64],
+    "vt_debug_prove_bvh": [I32, P, SZ, P, SZ, P, SZ, SZ, I32],
     "vt_reset": [P],
     "vt_engine_get_stats": [P, P],
     "vt_destroy": [P],

@@ -226,6 +226,41 @@ vt_status vt_debug_fail_device_allocation(int64_t nth) {
   });
 }
 
+vt_status vt_debug_prove_bvh(int32_t on_device, const uint32_t* binary_words, size_t binary_nodes,
+                             const uint32_t* wide_words, size_t wide_nodes, const float* records,
+                             size_t record_count, size_t triangle_count, int32_t stack_capacity) {
+  return guard([&] {
+    if ((binary_words && !binary_nodes) || (wide_words && !wide_nodes) || (record_count && !records))
+      fail(VT_ERR_INVALID_ARGUMENT, "words without a count, or a count without records");
+    if (stack_capacity <= 0) fail(VT_ERR_RANGE, "stack_capacity must be positive");
+    if (!on_device) {
+      BinaryBvhHost h;
+      h.nodes.resize(binary_words ? binary_nodes : 0);
+      if (binary_words) {
+        std::memcpy(h.nodes.data(), binary_words, binary_nodes * sizeof(BinaryNode));
+        validate_binary(h, (int64_t)triangle_count, stack_capacity);
+      }
+      if (wide_words)
+        validate_wide(wide_words, wide_nodes, records, record_count, 0, triangle_count, false, stack_capacity);
+      return;
+    }
+    cudaStream_t s = nullptr;
+    if (binary_words) {
+      ScratchBuffer<BinaryNode> nodes(binary_nodes, s);
+      VT_CUDA(cudaMemcpyAsync(nodes.ptr, binary_words, nodes.bytes(), cudaMemcpyHostToDevice, s));
+      prove_binary_gpu(nodes.ptr, binary_nodes, triangle_count, stack_capacity, s);
+    }
+    if (wide_words) {
+      ScratchBuffer<uint32_t> words(20 * wide_nodes, s);
+      ScratchBuffer<float> recs(std::max<size_t>(16 * record_count, 1), s);
+      VT_CUDA(cudaMemcpyAsync(words.ptr, wide_words, words.bytes(), cudaMemcpyHostToDevice, s));
+      if (record_count)
+        VT_CUDA(cudaMemcpyAsync(recs.ptr, records, 64 * record_count, cudaMemcpyHostToDevice, s));
+      prove_wide_gpu(words.ptr, wide_nodes, recs.ptr, record_count, triangle_count, stack_capacity, s);
+    }
+  });
+}
+
 vt_status vt_bvh_build(int32_t device, const float* positions, size_t position_words, const uint32_t* indices,
                        size_t index_words, const vt_bvh_build_options* options, vt_bvh** out_bvh) {
   return guard([&] {
