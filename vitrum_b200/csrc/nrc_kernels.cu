@@ -1,12 +1,12 @@
 // nrc_kernels.cu -- neural radiance cache kernels for sm_100a.
 //
 // k_nrc_infer   persistent; per tile of 128 queries: encode
-//               (hash grid + SH4 + surface features) into a swizzled fp16 tile, then six
+//               (hash grid + SH4 + surface features) into fp16 rows in TMEM, then six
 //               tcgen05.mma layers (M=128, N=64, K=64 as four K=16 steps) with
-//               the fp32 accumulator in TMEM, ReLU + fp16 repack in the epilogue
+//               A and the fp32 accumulator in TMEM, ReLU + fp16 repack in the epilogue
 //               between layers, prediction read from TMEM.
 // k_nrc_train   persistent; per tile: encode, forward keeping every layer's
-//               activations in shared memory, relative-L2 output gradient,
+//               activations in swizzled shared-memory tiles, relative-L2 output gradient,
 //               backward: per layer dW += G^T X (tensor core, accumulated across
 //               the CTA's tiles in TMEM) and dX = G W (tensor core), ReLU mask
 //               from the stored activations; the input gradient of the 32
@@ -191,14 +191,7 @@ __device__ __forceinline__ void scatter_level(const View& v, int l, const PointP
   }
 }
 
-// Shared-memory carve-up (dynamic, aligned to 1024 at run time).
-struct Smem {
-  uint8_t* w;        // 6 weight tiles
-  uint8_t* act;      // activation tiles
-  uint64_t* bar;
-  uint32_t* tmem_slot;
-};
-
+// The dynamic shared memory from its first 1024-byte boundary on.
 __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
   const uint32_t s = tc::smem_u32(p);
   return p + (((s + 1023u) & ~1023u) - s);
@@ -264,10 +257,11 @@ __device__ __forceinline__ bool group_and(uint32_t id, bool p) {
 __host__ __device__ constexpr uint32_t infer_cols(int t) { return t == 1 ? 128u : (t == 2 ? 256u : 512u); }
 
 // T tiles of 128 queries in flight per CTA, one per warpgroup (the MLP tile
-// knob): the warpgroups share the CTA's weight tiles and TMEM allocation (64
-// columns each) and run independently -- each encodes its tile (16 levels x 8
-// table gathers per query), issues its own MMA chain from its first thread and
-// waits on its own mbarrier -- so one tile's gathers overlap another's MMAs.
+// knob): the warpgroups share the CTA's weight tiles and TMEM allocation (96
+// columns each: 64 of accumulators, 32 of layer input) and run independently --
+// each encodes its tile (16 levels x 8 table gathers per query), issues its own
+// MMA chain from its first thread and waits on its own mbarrier -- so one tile's
+// gathers overlap another's MMAs.
 // The layer inputs are the MMAs' A operands in TMEM, written by the thread that owns
 // the row: shared memory holds the weights alone (50 KB instead of 66 to 114), and
 // what it gives up is L1 for the gathers that bound the kernel: 1,048,576 queries of

@@ -171,19 +171,18 @@ __device__ __forceinline__ uint32_t nibble_spread8(uint32_t m) {
   return m * 15u;
 }
 
-// Resident CTAs per SM the register budget is cut for (80 registers, spills
-// only around the out-of-line exact test).  Measured (B200) at 5 / 6 / 7 / 8 /
-// 9: the 1,048,576-ray query 1.01 / 0.98 / 1.01 / 1.14 / 1.42 ms, the box-room
-// frame 25.9 / 24.8 / 25.1 / 25.9 / 28.4 ms; the instanced frame 24.7 / 24.7 /
-// 25.5 ms at 5 / 6 / 7.
+// Resident CTAs per SM the register budget is cut for (80 registers).  Measured
+// (B200) at 5 / 6 / 7 / 8: the 1,048,576-ray query 914 / 854 / 862 / 884 us, the
+// box-room frame 24.6 / 23.0 / 22.6 / 22.7 ms, the instanced frame 22.0 / 21.0 /
+// 21.0 / 21.5 ms.
 constexpr int kTraceBlocks = 6;
 
 // Idle lanes a warp gathers before it refills them.  Setting a ray up costs
 // about as much as expanding a node and a warp of the box-room frame finishes
 // 4.4 rays per iteration: refilling every idle lane at once ran the set-up in
-// 94 % of the iterations for those few lanes.  Measured at 1 / 4 / 6 / 8 / 12:
-// box-room frame 27.2 / 26.3 / 26.0 / 25.9 / 26.1 ms, query 1.18 / 1.13 / 1.13 /
-// 1.14 / 1.16 ms (at 64 registers).
+// 94 % of the iterations for those few lanes.  Measured at 4 / 8 / 12: box-room
+// frame 23.5 / 23.0 / 23.2 ms, instanced frame 21.0 / 21.0 / 21.3 ms, query 840 /
+// 853 / 891 us.
 constexpr int kRefillLanes = 8;
 
 // The last rays of an occlusion query's warp whose pool is spent (single-level
@@ -193,8 +192,8 @@ constexpr int kRefillLanes = 8;
 // which moves to the group's first lane.  Any order finds the same answer.  Such a
 // launch ends with its longest rays, each some 600 dependent instructions a step
 // in the loop: 300,001 segments in a room of 262,146 triangles 236 -> 170 us,
-// 20,000 123 -> 81, 36,000 in one of 16,384 67 -> 51, 60,000 through 65,536 loose
-// triangles 140 -> 131.  Closest hits gained less (30,000 in the room 147 -> 121 us)
+// 20,000 124 -> 83, 30,000 in one of 16,384 69 -> 54, 30,000 through 65,536 loose
+// triangles 126 -> 121.  Closest hits gained less (30,000 in the room 147 -> 121 us)
 // and lost elsewhere (the loop beside it 2.7 % slower, 60,000 through loose triangles
 // 162 -> 172); waiting 8 to 32 iterations before the change was slower in both.
 constexpr int kTailRays = 4;
@@ -386,7 +385,7 @@ __global__ void __launch_bounds__(kBlock, kTraceBlocks)
   // rays per pool refill: small enough to spread short launches over all warps
   // (16 / 32 / 64: instanced frame 25.1 / 24.7 / 25.7 ms, box room 26.7 / 25.9 /
   // 25.5 ms, a 1,000-ray query 55 / 54 / 98 us)
-    constexpr uint32_t kChunk = 32;
+  constexpr uint32_t kChunk = 32;
 
   bool live = false, exhausted = false;
   uint32_t ray = 0, pool_next = 0, pool_end = 0;
@@ -473,7 +472,7 @@ __global__ void __launch_bounds__(kBlock, kTraceBlocks)
 #pragma unroll
       for (int j = 7; j >= 0; --j) {
         const uint32_t sel = (uint32_t)(j & 3);
-        // near and far plane of one axis as one packed f32x2 conversion and FMA
+        // near and far plane of one axis: one packed FMA of the two bytes as floats
         const uint64_t tx = slab2(j < 4 ? nx0 : nx1, j < 4 ? fx0 : fx1, sel, ax2, ox2);
         const uint64_t ty = slab2(j < 4 ? ny0 : ny1, j < 4 ? fy0 : fy1, sel, ay2, oy2);
         const uint64_t tz = slab2(j < 4 ? nz0 : nz1, j < 4 ? fz0 : fz1, sel, az2, oz2);
@@ -1068,10 +1067,10 @@ template <bool ANY>
 void launch_trace_t(const TraceArgs& a, cudaStream_t s) {
   if (a.n == 0) return;
   // Up to here eight lanes per ray win (k_trace_group); measured, k_trace / group:
-  // closest hits of 1,000 rays on 4,096 loose triangles 49 / 35 us, 12,000 on 65,536
-  // 129 / 111, 16,384 137 / 139, 16,384 in a room of 16,384 75 / 64, 44,000 81 / 115;
-  // occlusion of 12,000 in a room of 262,146 118 / 58 (with finish_occlusion 81 / 71
-  // at 20,000), 36,000 in one of 16,384 51 / 59, on loose triangles 120 / 169
+  // closest hits of 1,000 rays on 4,096 loose triangles 53 / 35 us, 20,000 56 / 64,
+  // 12,000 on 65,536 133 / 88, 16,384 140 / 122, 30,000 143 / 146, 16,384 in a room of
+  // 16,384 80 / 60, 44,000 85 / 96; occlusion of 12,000 in a room of 262,146 80 / 57,
+  // 44,000 in one of 16,384 55 / 61, 30,000 on loose triangles 120 / 132
   constexpr size_t kGroupRays = 16384;
   if (!a.insts && a.n <= kGroupRays && !a.stage_nodes) {
     const int stk = std::min(std::max(a.stack_depth, 4), kMaxStack);
